@@ -17,15 +17,9 @@ template <int KER>
 __device__ __forceinline__ double seg_normal_influence(const double x[3], const double nrm[3],
                                                        const double* y0, const double* y1,
                                                        double rc2) {
-    Vtx64<KER> a, b;
-    vtx64<KER>(x, y0[0], y0[1], y0[2], a);
-    vtx64<KER>(x, y1[0], y1[1], y1[2], b);
-    const double r0x = y1[0] - y0[0], r0y = y1[1] - y0[1], r0z = y1[2] - y0[2];
-    const double r0sq = r0x * r0x + r0y * r0y + r0z * r0z;
-    const double q = (KER == FJ_KERNEL_EPSILON) ? kEps * r0sq * r0sq : r0sq;
-    double k[3] = {0.0, 0.0, 0.0};
-    link64<KER>(a, b, 1.0, r0x, r0y, r0z, q, rc2, k);
-    return k[0] * nrm[0] + k[1] * nrm[1] + k[2] * nrm[2];  // jnp.dot(K, n_i)
+    double k[3];
+    segment64<KER>(x, y0, y1, rc2, k);
+    return (k[0] * nrm[0] + k[1] * nrm[1] + k[2] * nrm[2]) * kInv4Pi;  // jnp.dot(K, n_i)
 }
 
 __device__ __forceinline__ void mirror_pt(const MirrorPlane& mp, const double* z, double o[3]) {

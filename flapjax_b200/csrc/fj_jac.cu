@@ -44,19 +44,6 @@ __device__ __forceinline__ double ring_g(const double* gamma, int R, int C, int 
     return (k < 0 || l < 0 || k >= R || l >= C) ? 0.0 : gamma[(int64_t)k * C + l];
 }
 
-// K(x; y0 -> y1) with unit strength, the forward arithmetic of the sums.
-template <int KER>
-__device__ __forceinline__ void seg_velocity(const double x[3], const double y0[3], const double y1[3], double rc2,
-                                             double acc[3]) {
-    Vtx64<KER> a, b;
-    vtx64<KER>(x, y0[0], y0[1], y0[2], a);
-    vtx64<KER>(x, y1[0], y1[1], y1[2], b);
-    const double r0x = y1[0] - y0[0], r0y = y1[1] - y0[1], r0z = y1[2] - y0[2];
-    const double r0sq = r0x * r0x + r0y * r0y + r0z * r0z;
-    const double q = KER == FJ_KERNEL_EPSILON ? kEps * r0sq * r0sq : r0sq;
-    link64<KER>(a, b, 1.0, r0x, r0y, r0z, q, rc2, acc);
-}
-
 template <int KER, bool NRM>
 __global__ void __launch_bounds__(kJacBlock) ring_influence_kernel(const double* __restrict__ tgt,
                                                                    const double* __restrict__ nrm, int64_t nt,
@@ -88,13 +75,13 @@ __global__ void __launch_bounds__(kJacBlock) ring_influence_kernel(const double*
         const double x[3] = {tgt[t * 3 + 0], tgt[t * 3 + 1], tgt[t * 3 + 2]};
         double v[3] = {0.0, 0.0, 0.0};
         for (int img = 0; img < (mirror ? 2 : 1); ++img) {
-            double m0[3] = {0.0, 0.0, 0.0}, m1[3] = {0.0, 0.0, 0.0}, n0[3] = {0.0, 0.0, 0.0}, n1[3] = {0.0, 0.0, 0.0};
-            seg_velocity<KER>(x, p[img][0], p[img][2], rc2, m0);  // M[k,l]
-            seg_velocity<KER>(x, p[img][1], p[img][3], rc2, m1);  // M[k,l+1]
-            seg_velocity<KER>(x, p[img][2], p[img][3], rc2, n1);  // N[k+1,l]
-            seg_velocity<KER>(x, p[img][0], p[img][1], rc2, n0);  // N[k,l]
+            double m0[3], m1[3], n0[3], n1[3];
+            segment64<KER>(x, p[img][0], p[img][2], rc2, m0);  // M[k,l]
+            segment64<KER>(x, p[img][1], p[img][3], rc2, m1);  // M[k,l+1]
+            segment64<KER>(x, p[img][2], p[img][3], rc2, n1);  // N[k+1,l]
+            segment64<KER>(x, p[img][0], p[img][1], rc2, n0);  // N[k,l]
             const double sg = img ? -1.0 : 1.0;
-            for (int d = 0; d < 3; ++d) v[d] += sg * ((m0[d] - m1[d]) + (n1[d] - n0[d]));
+            for (int d = 0; d < 3; ++d) v[d] += sg * kInv4Pi * ((m0[d] - m1[d]) + (n1[d] - n0[d]));
         }
         if (NRM) {
             out[t * ld + r] = v[0] * nrm[t * 3 + 0] + v[1] * nrm[t * 3 + 1] + v[2] * nrm[t * 3 + 2];

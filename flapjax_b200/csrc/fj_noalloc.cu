@@ -125,6 +125,8 @@ extern "C" FJ_API int fj_vind_noalloc(const double* d_targets, int64_t n_targets
     const int64_t fit = (int64_t)((kNoAllocScratchBytes - stream_bytes) / part_per_split);
     int n_split = choose_split(n_targets, n_elem, precision);
     if (n_split > fit) n_split = (int)fit;
+    const int n_sub = choose_sub(n_targets, n_elem, n_split, precision, choose_tile(n_targets, n_elem, precision),
+                                 std::min<int64_t>(fit, part_bound(n_targets, n_elem, precision)));
     if (precision == FJ_PREC_FP64)
         FJ_TRY(pack_stream64(pa, (Elem64*)st, s));
     else
@@ -135,8 +137,9 @@ extern "C" FJ_API int fj_vind_noalloc(const double* d_targets, int64_t n_targets
     j.stream = st;
     j.n_elem = n_elem;
     j.n_split = n_split;
+    j.n_sub = n_sub;
     j.part = part;
     j.n_links = n_links;
     FJ_TRY(vind_launch(j, precision, kernel, r_cut, s));
-    return reduce_partials(part, n_split, n_targets, d_v_out, 0, 1.0, s);
+    return reduce_partials(part, n_split * n_sub, n_targets, d_v_out, 0, 1.0, s);
 }

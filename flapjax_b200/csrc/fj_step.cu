@@ -966,7 +966,7 @@ static int make_plan(const fj_case_config* cfg, void* ws, size_t ws_bytes, Plan&
     const int64_t sets[3] = {L.wto[ns], L.fo[ns], L.po[ns]};
     for (int64_t nt : sets) {
         if (nt == 0) continue;
-        part = std::max<int64_t>(part, (int64_t)split_bound(nt, stream, cfg->precision) * nt * 3);
+        part = std::max<int64_t>(part, (int64_t)part_bound(nt, stream, cfg->precision) * nt * 3);
     }
     p.part_elems = part;
 
@@ -1091,12 +1091,14 @@ static int vind_sum(const Plan& p, const double* targets, int64_t nt, int64_t n_
     j.stream = p.stream;
     j.n_elem = n_elem;
     j.n_split = choose_split(nt, n_elem, p.cfg.precision);
+    j.n_sub = choose_sub(nt, n_elem, j.n_split, p.cfg.precision, choose_tile(nt, n_elem, p.cfg.precision),
+                         p.part_elems / (nt * 3));
     j.part = p.part;
     j.n_links = n_links;
     j.out = out;
     if ((int64_t)j.n_split * nt * 3 > p.part_elems) return fail(FJ_ERR_NOMEM, "partial buffer too small");
     FJ_TRY(vind_launch(j, p.cfg.precision, p.cfg.kernel, p.cfg.r_cut, s));
-    return reduce_partials(p.part, j.n_split, nt, out, 0, 1.0, s);
+    return reduce_partials(p.part, j.n_split * j.n_sub, nt, out, 0, 1.0, s);
 }
 
 static void fill_aic_args(const Plan& p, AicArgs& a, const double* zeta, const double* c, const double* nc,
@@ -1577,6 +1579,7 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
             const int64_t cap = part_elems[j.part] / std::max<int64_t>(1, j.n_targets * 3);
             if (cap < 1) return fail(FJ_ERR_NOMEM, "partial buffer too small for %lld targets", (long long)j.n_targets);
             j.n_split = (int)std::min<int64_t>(j.n_split, cap);
+            j.n_sub = 1;
         }
     // one tile (targets per thread) per FP32 launch: the autotuned choice of its largest job
     auto phase_tile = [&](const std::vector<VindJob>& jobs) {
@@ -1592,11 +1595,23 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
         return tile;
     };
     const int tf = phase_tile(jf), tr = phase_tile(jr), tfo = phase_tile(jfo);
+    // one case: its splits alone leave SMs idle where it is small
+    if (K == 1) {
+        auto cut = [&](std::vector<VindJob>& jobs, int prec, int tile) {
+            for (VindJob& j : jobs)
+                j.n_sub = choose_sub(j.n_targets, j.n_elem, j.n_split, prec, tile,
+                                     part_elems[j.part] / std::max<int64_t>(1, j.n_targets * 3));
+        };
+        cut(jf, precision, tf);
+        cut(jr, precision, tr);
+        cut(jfo, precision, tfo);
+        cut(jrn, FJ_PREC_FP64, 0);
+    }
     auto fill_cta = [&](const std::vector<VindJob>& jobs, size_t off, int prec, int tile) {
         int64_t* c0 = (int64_t*)(h.data() + off);
         c0[0] = 0;
         for (size_t q = 0; q < jobs.size(); ++q)
-            c0[q + 1] = c0[q] + vind_ctas(jobs[q].n_targets, jobs[q].n_split, prec, tile);
+            c0[q + 1] = c0[q] + vind_ctas(jobs[q].n_targets, jobs[q].n_split * jobs[q].n_sub, prec, tile);
         return std::vector<int64_t>(c0, c0 + jobs.size() + 1);
     };
     const std::vector<int64_t> cf = fill_cta(jf, tl.cta_free, precision, tf),
@@ -2145,7 +2160,7 @@ int fj_biot_savart(const double* d_x, const double* d_y, int64_t n_pairs, int ke
 }
 
 static int vind_plan(int64_t n_targets, const int* rows, const int* cols, int n_lattices, int mirror, int precision,
-                     int64_t& n_elem, int& n_split, size_t& bytes) {
+                     int64_t& n_elem, int& n_part, size_t& bytes) {
     if (n_targets < 0 || n_lattices < 0 || n_lattices > FJ_MAX_SURF * 2)
         return fail(FJ_ERR_SHAPE, "vind: n_targets=%lld n_lattices=%d", (long long)n_targets, n_lattices);
     if (precision != FJ_PREC_FP64 && precision != FJ_PREC_MIXED) return fail(FJ_ERR_UNSUPPORTED, "precision %d", precision);
@@ -2154,10 +2169,10 @@ static int vind_plan(int64_t n_targets, const int* rows, const int* cols, int n_
         if (rows[i] < 0 || cols[i] < 0) return fail(FJ_ERR_SHAPE, "vind: lattice %d has rows=%d cols=%d", i, rows[i], cols[i]);
         n_elem += (mirror ? 2 : 1) * stream_len(rows[i], cols[i]);
     }
-    n_split = split_bound(std::max<int64_t>(n_targets, 1), n_elem, precision);
+    n_part = part_bound(std::max<int64_t>(n_targets, 1), n_elem, precision);
     Arena a(nullptr, 0);
     a.carve<Elem64>(n_elem);
-    a.carve<double>((int64_t)n_split * std::max<int64_t>(n_targets, 1) * 3);
+    a.carve<double>((int64_t)n_part * std::max<int64_t>(n_targets, 1) * 3);
     bytes = a.used + 256;
     return FJ_OK;
 }
@@ -2228,12 +2243,13 @@ int fj_vind(const double* d_targets, int64_t n_targets, const double* const* d_z
     j.stream = st;
     j.n_elem = ne;
     j.n_split = std::min(sp, choose_split(n_targets, ne, precision));
+    j.n_sub = choose_sub(n_targets, ne, j.n_split, precision, choose_tile(n_targets, ne, precision), sp);
     j.part = part;
     j.out = d_v_out;
     j.n_links = 0;
     for (int i = 0; i < n_lattices; ++i) j.n_links += (mirror ? 2 : 1) * lattice_links(rows[i], cols[i]);
     FJ_TRY(vind_launch(j, precision, kernel, r_cut, s));
-    return reduce_partials(part, j.n_split, n_targets, d_v_out, 0, 1.0, s);
+    return reduce_partials(part, j.n_split * j.n_sub, n_targets, d_v_out, 0, 1.0, s);
 }
 
 int fj_aic_workspace_size(const int* m, const int* n, int n_surf, size_t* bytes) {

@@ -76,7 +76,7 @@ ShapeWs shape_ws(int precision, int64_t n_targets, int64_t n_elem) {
     w.zeta = (size_t)(rows + 1) * (cols + 1) * 3;
     w.gamma = (size_t)rows * cols;
     w.stream = (size_t)ne;
-    w.part = (size_t)split_bound(n_targets, ne, precision) * n_targets * 3;
+    w.part = (size_t)part_bound(n_targets, ne, precision) * n_targets * 3;
     w.out = (size_t)n_targets * 3;
     a.carve<double>(w.targets);
     a.carve<double>(w.zeta);
@@ -132,8 +132,8 @@ int fj_autotune_vind(int precision, int kernel, double r_cut, const int64_t* n_t
         double* zeta = a.carve<double>((size_t)(rows + 1) * (cols + 1) * 3);
         double* gamma = a.carve<double>((size_t)rows * cols);
         void* strm = precision == FJ_PREC_FP64 ? (void*)a.carve<Elem64>(ne) : (void*)a.carve<Elem32>(ne);
-        const int bound = split_bound(nt, ne, precision);
-        double* part = a.carve<double>((size_t)bound * nt * 3);
+        const int bound = split_bound(nt, ne, precision), parts = part_bound(nt, ne, precision);
+        double* part = a.carve<double>((size_t)parts * nt * 3);
         double* out = a.carve<double>((size_t)nt * 3);
         const int64_t nv = (int64_t)(rows + 1) * (cols + 1);
         tune_lattice_kernel<<<(unsigned)((nv + 255) / 256), 256, 0, s>>>(zeta, gamma, rows, cols);
@@ -165,13 +165,14 @@ int fj_autotune_vind(int precision, int kernel, double r_cut, const int64_t* n_t
         }
         for (const auto& trial : trials) {
             const int sp = trial.first, tile = trial.second;
-            VindJob job{targets, nt, strm, ne, sp, part, ne, out};
+            const int sub = choose_sub(nt, ne, sp, precision, tile, parts);
+            VindJob job{targets, nt, strm, ne, sp, sub, part, ne, out, 0};
             float t = 1e30f;
             for (int rep = 0; rep < 4 && st == FJ_OK; ++rep) {
                 float ms = 0.0f;
                 st = cuda_status(cudaEventRecord(e0, s), "autotune event");
                 if (st == FJ_OK) st = vind_launch(job, precision, kernel, r_cut, s, tile);
-                if (st == FJ_OK) st = reduce_partials(part, sp, nt, out, 0, 1.0, s);
+                if (st == FJ_OK) st = reduce_partials(part, sp * sub, nt, out, 0, 1.0, s);
                 if (st == FJ_OK) st = cuda_status(cudaEventRecord(e1, s), "autotune event");
                 if (st == FJ_OK) st = cuda_status(cudaEventSynchronize(e1), "autotune sync");
                 if (st == FJ_OK) st = cuda_status(cudaEventElapsedTime(&ms, e0, e1), "autotune timing");

@@ -323,19 +323,44 @@ int pack_stream32(const PackArgs& a, Elem32* out, cudaStream_t s) {
 }
 
 // ------------------------------------------------------------------------------------
-// FP64 sum: the reference's kernels, evaluated on chains.
+// The stream's cuts.  A sum's stream is cut into n_split splits of `per` links, and each
+// split into n_sub pieces, one CTA per (target tile, piece), each with partials of its own.
+// A piece starts on a multiple of kFold links from its split's start, so the FP32 sum's
+// folds (16 links summed in FP32, then added in FP64) are those of the whole split: the
+// number of pieces changes only the order of FP64 additions.
 // ------------------------------------------------------------------------------------
 constexpr int kBlock = 128;  // threads per CTA == staged elements per chunk
+constexpr int kFold = 16;    // elements per FP32 partial sum (even: the ping-pong takes pairs)
+constexpr int kFold64 = 8;   // the FP64 sum's smallest piece
 
+struct PieceRange {
+    int64_t e0, vend;  // links [e0, vend), vertices e0 .. vend
+};
+
+__host__ __device__ __forceinline__ int64_t piece_len(int64_t n_elem, int n_split, int n_sub, int fold) {
+    const int64_t per = (n_elem + n_split - 1) / n_split;
+    return ((per + fold - 1) / fold + n_sub - 1) / n_sub * fold;
+}
+
+__device__ __forceinline__ PieceRange piece_range(int64_t n_elem, int n_split, int n_sub, int fold, int piece) {
+    const int64_t per = (n_elem + n_split - 1) / n_split, len = piece_len(n_elem, n_split, n_sub, fold);
+    const int64_t s0 = (int64_t)(piece / n_sub) * per;
+    const int64_t s1 = min(n_elem, s0 + per);
+    PieceRange r;
+    r.e0 = s0 + (int64_t)(piece % n_sub) * len;
+    r.vend = min(min(s1, r.e0 + len), n_elem - 1);
+    return r;
+}
+
+// ------------------------------------------------------------------------------------
+// FP64 sum: the reference's kernels, evaluated on chains.
+// ------------------------------------------------------------------------------------
 template <int KER, int T>
 __device__ __forceinline__ void vind64_body(const double* __restrict__ tgt, int64_t n_t,
-                                            const Elem64* __restrict__ st, int64_t n_elem, int n_split,
-                                            double* __restrict__ part, double rc2, int64_t tile, int split) {
+                                            const Elem64* __restrict__ st, int64_t n_elem, int n_split, int n_sub,
+                                            double* __restrict__ part, double rc2, int64_t tile, int piece) {
     __shared__ Elem64 sh[kBlock];
-    const int64_t per = (n_elem + n_split - 1) / n_split;
-    const int64_t e0 = (int64_t)split * per;
-    const int64_t e1 = min(n_elem, e0 + per);  // links [e0, e1)
-    const int64_t vend = min(e1, n_elem - 1);  // last vertex needed
+    const PieceRange pr = piece_range(n_elem, n_split, n_sub, kFold64, piece);
 
     double x[T][3];
     int64_t ti[T];
@@ -351,25 +376,31 @@ __device__ __forceinline__ void vind64_body(const double* __restrict__ tgt, int6
 #pragma unroll
     for (int j = 0; j < T; ++j) acc[j][0] = acc[j][1] = acc[j][2] = 0.0;
 
-    if (e0 < e1) {
+    if (pr.e0 < pr.vend) {
         Vtx64<KER> prev[T];
-        Elem64 pl = st[e0];
+        Elem64 pl = st[pr.e0];
+        if (KER == FJ_KERNEL_CUTOFF) pl.q *= rc2;
 #pragma unroll
         for (int j = 0; j < T; ++j) vtx64<KER>(x[j], pl.x, pl.y, pl.z, prev[j]);
-        for (int64_t c0 = e0 + 1; c0 <= vend; c0 += kBlock) {
-            const int cnt = (int)min((int64_t)kBlock, vend + 1 - c0);
+        for (int64_t c0 = pr.e0 + 1; c0 <= pr.vend; c0 += kBlock) {
+            const int cnt = (int)min((int64_t)kBlock, pr.vend + 1 - c0);
             __syncthreads();
-            if (threadIdx.x < cnt) sh[threadIdx.x] = st[c0 + threadIdx.x];
+            if (threadIdx.x < cnt) {
+                Elem64 e = st[c0 + threadIdx.x];
+                if (KER == FJ_KERNEL_CUTOFF) e.q *= rc2;  // (a break keeps its sign)
+                sh[threadIdx.x] = e;
+            }
             __syncthreads();
+#pragma unroll 2
             for (int i = 0; i < cnt; ++i) {
                 const Elem64 cur = sh[i];
+                Vtx64<KER> v[T];
 #pragma unroll
-                for (int j = 0; j < T; ++j) {
-                    Vtx64<KER> v;
-                    vtx64<KER>(x[j], cur.x, cur.y, cur.z, v);
-                    if (pl.q >= 0.0) link64<KER>(prev[j], v, pl.g, pl.r0x, pl.r0y, pl.r0z, pl.q, rc2, acc[j]);
-                    prev[j] = v;
-                }
+                for (int j = 0; j < T; ++j) vtx64<KER>(x[j], cur.x, cur.y, cur.z, v[j]);
+                if (__double2hiint(pl.q) >= 0)  // not a chain's last vertex
+                    link64<KER, T>(prev, v, pl.g, pl.r0x, pl.r0y, pl.r0z, pl.q, rc2, acc);
+#pragma unroll
+                for (int j = 0; j < T; ++j) prev[j] = v[j];
                 pl = cur;
             }
         }
@@ -377,18 +408,21 @@ __device__ __forceinline__ void vind64_body(const double* __restrict__ tgt, int6
 #pragma unroll
     for (int j = 0; j < T; ++j) {
         if (ti[j] < n_t) {
-            double* o = part + ((int64_t)split * n_t + ti[j]) * 3;
-            o[0] = acc[j][0];
-            o[1] = acc[j][1];
-            o[2] = acc[j][2];
+            double* o = part + ((int64_t)piece * n_t + ti[j]) * 3;
+            o[0] = acc[j][0] * kInv4Pi;
+            o[1] = acc[j][1] * kInv4Pi;
+            o[2] = acc[j][2] * kInv4Pi;
         }
     }
 }
 
+// Four resident CTAs per SM (registers capped at 128): 3 and 5 were 3 % and 0.5 % slower on
+// the 16 x 128 free wake, one or four targets per thread 8 and 5 %.
+constexpr int kMinCtas64 = 4;
 template <int KER, int T>
-__global__ void __launch_bounds__(kBlock) vind64_kernel(VindJob job, double rc2) {
-    vind64_body<KER, T>(job.targets, job.n_targets, (const Elem64*)job.stream, job.n_elem, job.n_split, job.part, rc2,
-                        blockIdx.x, blockIdx.y);
+__global__ void __launch_bounds__(kBlock, kMinCtas64) vind64_kernel(VindJob job, double rc2) {
+    vind64_body<KER, T>(job.targets, job.n_targets, (const Elem64*)job.stream, job.n_elem, job.n_split, job.n_sub,
+                        job.part, rc2, blockIdx.x, blockIdx.y);
 }
 
 // ------------------------------------------------------------------------------------
@@ -441,8 +475,6 @@ template <int T>
 struct MinCtas32 {
     static constexpr int value = T == 2 ? kMinCtas32 : kMinCtas32Wide;
 };
-constexpr int kFold = 16;  // elements per FP32 partial sum (even: the ping-pong takes pairs)
-
 __device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
 
 // MUFU approximations with flush-to-zero (PTX rsqrt.approx.ftz / rcp.approx.ftz): the
@@ -531,16 +563,14 @@ __device__ __forceinline__ void stage_dup(const float4* __restrict__ s4, int64_t
 
 template <int KER, int T>
 __device__ __forceinline__ void vind32_body(const double* __restrict__ tgt, int64_t n_t,
-                                            const Elem32* __restrict__ st, int64_t n_elem, int n_split,
-                                            double* __restrict__ part, int64_t tile, int split) {
+                                            const Elem32* __restrict__ st, int64_t n_elem, int n_split, int n_sub,
+                                            double* __restrict__ part, int64_t tile, int piece) {
     static_assert(T % 2 == 0, "targets come in pairs");
     constexpr int P = T / 2;
     // slot 0: the element before the chunk (owner of the chunk's first link); 1..cnt: chunk
     __shared__ float4 sh[(kBlock + 1) * kDup];
-    const int64_t per = (n_elem + n_split - 1) / n_split;
-    const int64_t e0 = (int64_t)split * per;
-    const int64_t e1 = min(n_elem, e0 + per);
-    const int64_t vend = min(e1, n_elem - 1);
+    const PieceRange pr = piece_range(n_elem, n_split, n_sub, kFold, piece);
+    const int64_t e0 = pr.e0, vend = pr.vend;
 
     // pack p holds targets j = 2p (.x) and 2p+1 (.y); target j is threadIdx.x + j kBlock
     float2 xh[P][3], xl[P][3];
@@ -561,7 +591,7 @@ __device__ __forceinline__ void vind32_body(const double* __restrict__ tgt, int6
 #pragma unroll
     for (int j = 0; j < T; ++j) acc[j][0] = acc[j][1] = acc[j][2] = 0.0;
 
-    if (e0 < e1) {
+    if (e0 < vend) {
         const float4* s4 = reinterpret_cast<const float4*>(st);
         // A: vertex of the element owning the next link; B: the one after (ping-pong)
         Vtx32x2 A[P], B[P];
@@ -621,7 +651,7 @@ __device__ __forceinline__ void vind32_body(const double* __restrict__ tgt, int6
 #pragma unroll
     for (int j = 0; j < T; ++j) {
         if (ti[j] < n_t) {
-            double* o = part + ((int64_t)split * n_t + ti[j]) * 3;
+            double* o = part + ((int64_t)piece * n_t + ti[j]) * 3;
             o[0] = acc[j][0];
             o[1] = acc[j][1];
             o[2] = acc[j][2];
@@ -631,8 +661,8 @@ __device__ __forceinline__ void vind32_body(const double* __restrict__ tgt, int6
 
 template <int KER, int T>
 __global__ void __launch_bounds__(kBlock, MinCtas32<T>::value) vind32_kernel(VindJob job) {
-    vind32_body<KER, T>(job.targets, job.n_targets, (const Elem32*)job.stream, job.n_elem, job.n_split, job.part,
-                        blockIdx.x, blockIdx.y);
+    vind32_body<KER, T>(job.targets, job.n_targets, (const Elem32*)job.stream, job.n_elem, job.n_split, job.n_sub,
+                        job.part,                         blockIdx.x, blockIdx.y);
 }
 
 // Many jobs in one launch: CTA b belongs to the job j with cta0[j] <= b < cta0[j+1];
@@ -662,13 +692,13 @@ __global__ void __launch_bounds__(kBlock, MinCtas32<T>::value) vind32_jobs_kerne
         const VindJob job = jobs[j];
         const int64_t local = b - cta0[j];
         const int64_t ctas_x = (job.n_targets + (int64_t)kBlock * T - 1) / ((int64_t)kBlock * T);
-        vind32_body<KER, T>(job.targets, job.n_targets, (const Elem32*)job.stream, job.n_elem, job.n_split, job.part,
-                            local % ctas_x, (int)(local / ctas_x));
+        vind32_body<KER, T>(job.targets, job.n_targets, (const Elem32*)job.stream, job.n_elem, job.n_split, job.n_sub,
+                        job.part, local % ctas_x, (int)(local / ctas_x));
     }
 }
 
 template <int KER, int T>
-__global__ void __launch_bounds__(kBlock) vind64_jobs_kernel(const VindJob* __restrict__ jobs,
+__global__ void __launch_bounds__(kBlock, kMinCtas64) vind64_jobs_kernel(const VindJob* __restrict__ jobs,
                                                              const int64_t* __restrict__ cta0, int n_jobs,
                                                              double rc2) {
     const int64_t total = cta0[n_jobs];
@@ -677,45 +707,63 @@ __global__ void __launch_bounds__(kBlock) vind64_jobs_kernel(const VindJob* __re
         const VindJob job = jobs[j];
         const int64_t local = b - cta0[j];
         const int64_t ctas_x = (job.n_targets + (int64_t)kBlock * T - 1) / ((int64_t)kBlock * T);
-        vind64_body<KER, T>(job.targets, job.n_targets, (const Elem64*)job.stream, job.n_elem, job.n_split, job.part,
-                            rc2, local % ctas_x, (int)(local / ctas_x));
+        vind64_body<KER, T>(job.targets, job.n_targets, (const Elem64*)job.stream, job.n_elem, job.n_split, job.n_sub,
+                        job.part, rc2, local % ctas_x, (int)(local / ctas_x));
     }
 }
 
-__global__ void reduce_partials_kernel(const double* __restrict__ part, int n_split, int64_t n3,
-                                       double* __restrict__ out, int accumulate, double scale) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n3) return;
+// The partials of one sum, added in a fixed order: 16 lanes per output take every
+// sixteenth partial each (16 outputs of 8 bytes side by side), eight loads in flight, then
+// lane 0 adds the sixteen.  Latency-bound: a few dependent rounds of loads.
+constexpr int kRedOut = 16, kRedLanes = 16;
+
+__device__ __forceinline__ void reduce_outputs(const double* __restrict__ part, int n_part, int64_t n3,
+                                               double* __restrict__ out, int accumulate, double scale) {
+    __shared__ double sh[kRedLanes][kRedOut];
+    const int o = threadIdx.x % kRedOut, l = threadIdx.x / kRedOut;
+    const int64_t i = (int64_t)blockIdx.x * kRedOut + o;
     double s = 0.0;
-    for (int k = 0; k < n_split; ++k) s += part[(int64_t)k * n3 + i];
-    s *= scale;
-    out[i] = accumulate ? out[i] + s : s;
+    if (i < n3) {
+#pragma unroll 8
+        for (int k = l; k < n_part; k += kRedLanes) s += part[(int64_t)k * n3 + i];
+    }
+    sh[l][o] = s;
+    __syncthreads();
+    if (l == 0 && i < n3) {
+#pragma unroll
+        for (int k = 1; k < kRedLanes; ++k) s += sh[k][o];
+        s *= scale;
+        out[i] = accumulate ? out[i] + s : s;
+    }
 }
 
-__global__ void reduce_jobs_kernel(const VindJob* __restrict__ jobs) {
+__global__ void __launch_bounds__(kRedOut * kRedLanes)
+    reduce_partials_kernel(const double* __restrict__ part, int n_part, int64_t n3, double* __restrict__ out,
+                           int accumulate, double scale) {
+    reduce_outputs(part, n_part, n3, out, accumulate, scale);
+}
+
+__global__ void __launch_bounds__(kRedOut * kRedLanes) reduce_jobs_kernel(const VindJob* __restrict__ jobs) {
     const VindJob& J = jobs[blockIdx.y];
     const int64_t n3 = J.n_targets * 3;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n3) return;
-    double sacc = 0.0;
-    for (int k = 0; k < J.n_split; ++k) sacc += J.part[(int64_t)k * n3 + i];
-    J.out[i] = J.accumulate ? J.out[i] + sacc : sacc;
+    if ((int64_t)blockIdx.x * kRedOut >= n3) return;
+    reduce_outputs(J.part, J.n_split * J.n_sub, n3, J.out, J.accumulate, 1.0);
 }
 
 int reduce_jobs(const VindJob* d_jobs, int n_jobs, int64_t max_targets, cudaStream_t s) {
     if (n_jobs == 0 || max_targets == 0) return FJ_OK;
-    dim3 g((unsigned)((max_targets * 3 + 255) / 256), (unsigned)n_jobs);
-    reduce_jobs_kernel<<<g, 256, 0, s>>>(d_jobs); note_launch();
+    dim3 g((unsigned)((max_targets * 3 + kRedOut - 1) / kRedOut), (unsigned)n_jobs);
+    reduce_jobs_kernel<<<g, kRedOut * kRedLanes, 0, s>>>(d_jobs); note_launch();
     FJ_LAUNCH_CHECK("reduce_jobs_kernel");
     return FJ_OK;
 }
 
-int reduce_partials(const double* part, int n_split, int64_t n_targets, double* out, int accumulate,
+int reduce_partials(const double* part, int n_part, int64_t n_targets, double* out, int accumulate,
                     double scale, cudaStream_t s) {
     const int64_t n3 = n_targets * 3;
     if (n3 == 0) return FJ_OK;
-    reduce_partials_kernel<<<(unsigned)((n3 + 255) / 256), 256, 0, s>>>(part, n_split, n3, out,
-                                                                         accumulate, scale); note_launch();
+    reduce_partials_kernel<<<(unsigned)((n3 + kRedOut - 1) / kRedOut), kRedOut * kRedLanes, 0, s>>>(
+        part, n_part, n3, out, accumulate, scale); note_launch();
     FJ_LAUNCH_CHECK("reduce_partials_kernel");
     return FJ_OK;
 }
@@ -756,6 +804,52 @@ int split_bound(int64_t n_targets, int64_t n_elem_max, int precision) {
     const int64_t ctas = std::max<int64_t>(1, (n_targets + (int64_t)kBlock * T - 1) / ((int64_t)kBlock * T));
     const int64_t cap = (4ll * 160 * 16 + ctas - 1) / ctas;  // 4 waves of 160 SMs x 16 CTAs
     return (int)std::max<int64_t>(1, std::min<int64_t>({1024, cap, std::max<int64_t>(1, n_elem_max / 256)}));
+}
+
+// Partials a sum of up to n_elem_max elements may have (workspace sizing): the splits, or,
+// for few targets, the pieces of one wave of six CTAs on each of 148 SMs.
+constexpr int kPieceWave = 888;
+
+int part_bound(int64_t n_targets, int64_t n_elem_max, int precision) {
+    const int T = precision == FJ_PREC_FP64 ? kT64 : kT32, fold = precision == FJ_PREC_FP64 ? kFold64 : kFold;
+    const int64_t ctas = std::max<int64_t>(1, (n_targets + (int64_t)kBlock * T - 1) / ((int64_t)kBlock * T));
+    const int64_t pieces = std::min<int64_t>(kPieceWave / ctas, n_elem_max / fold);
+    return (int)std::max<int64_t>(split_bound(n_targets, n_elem_max, precision), pieces);
+}
+
+// Pieces per split.  A CTA's time is its links plus a fixed start (targets, first chunk,
+// partials: kStart links' worth).  With few CTAs a sum is latency-bound: the links of a
+// piece run one after the other, so more and shorter pieces win until every SM holds a
+// wave; beyond, whole waves of CTAs take turns on the FP pipe, and a cut only pays where it
+// evens out the last one.  Each extra partial costs the reduction about kReduce links.
+// Measured (8 x 32 wing, 64 wake rows, epsilon kernel, one step's larger sum): FP64 107 us in
+// 19 splits -> 14 us in 304 pieces; FP32 34 -> 8 us.
+int choose_sub(int64_t n_targets, int64_t n_elem, int n_split, int precision, int tile, int64_t max_part) {
+    query_occupancy();
+    const bool fp64 = precision == FJ_PREC_FP64;
+    const int T = fp64 ? kT64 : (tile ? tile : kT32), fold = fp64 ? kFold64 : kFold;
+    const int64_t per = (n_elem + n_split - 1) / n_split;
+    const int64_t max_sub = std::min<int64_t>({max_part / std::max(n_split, 1), (per + fold - 1) / fold, 4096});
+    const int64_t ctas = (n_targets + (int64_t)kBlock * T - 1) / ((int64_t)kBlock * T) * n_split;
+    const int res = fp64 ? g_res64 : (T == kT32Wide ? g_res32w : g_res32);
+    const int64_t wave = (int64_t)g_sms * res;
+    constexpr double kStart = 12.0, kReduce = 0.25, kSaturate = 0.75;
+    int best = 1;
+    double best_cost = 0.0;
+    for (int64_t sub = 1; sub <= max_sub; ++sub) {
+        const double len = (double)piece_len(n_elem, n_split, (int)sub, fold) + kStart;
+        const int64_t total = ctas * sub;
+        // CTAs one SM runs in turn, its pipes full from kSaturate of its resident CTAs on
+        const double turns = std::max((double)((total + g_sms - 1) / g_sms),
+                                      kSaturate * res * (double)((total + wave - 1) / wave));
+        const double cost = turns * len + kReduce * (double)(n_split * sub);
+        if (sub == 1 || cost < 0.98 * best_cost) {
+            best = (int)sub;
+            best_cost = cost;
+        }
+        if (total > 8 * wave) break;
+    }
+    return best;
 }
 
 // Autotuned splits (fj_autotune_vind): published once per tuning as a whole new table,
@@ -827,10 +921,10 @@ int vind_launch(const VindJob& job, int precision, int kernel, double r_cut, cud
     if (job.n_targets == 0) return FJ_OK;
     query_occupancy();
     const int T = precision == FJ_PREC_FP64 ? kT64 : (tile ? tile : choose_tile(job.n_targets, job.n_elem, precision));
-    if (T != kT32 && T != kT32Wide) return fail(FJ_ERR_SHAPE, "vind: tile %d (2 or 4 targets per thread)", T);
+    if (precision != FJ_PREC_FP64 && T != kT32 && T != kT32Wide) return fail(FJ_ERR_SHAPE, "vind: tile %d (2 or 4 targets per thread)", T);
     const int64_t gx = (job.n_targets + (int64_t)kBlock * T - 1) / ((int64_t)kBlock * T);
-    if (gx > 0x7fffffff || job.n_split > 65535) return fail(FJ_ERR_SHAPE, "vind: grid too large");
-    dim3 grid((unsigned)gx, (unsigned)job.n_split);
+    if (gx > 0x7fffffff || (int64_t)job.n_split * job.n_sub > 65535) return fail(FJ_ERR_SHAPE, "vind: grid too large");
+    dim3 grid((unsigned)gx, (unsigned)(job.n_split * job.n_sub));
     const int prof = prof_start(s);
     if (precision == FJ_PREC_FP64) {
         const double rc2 = r_cut * r_cut;
@@ -868,9 +962,9 @@ int vind_launch(const VindJob& job, int precision, int kernel, double r_cut, cud
     return FJ_OK;
 }
 
-int64_t vind_ctas(int64_t n_targets, int n_split, int precision, int tile) {
+int64_t vind_ctas(int64_t n_targets, int n_part, int precision, int tile) {
     const int T = precision == FJ_PREC_FP64 ? kT64 : (tile ? tile : kT32);
-    return (n_targets + (int64_t)kBlock * T - 1) / ((int64_t)kBlock * T) * n_split;
+    return (n_targets + (int64_t)kBlock * T - 1) / ((int64_t)kBlock * T) * n_part;
 }
 
 int vind_launch_jobs(const VindJob* d_jobs, const int64_t* d_cta0, int n_jobs, int64_t total_ctas, double pairs,
@@ -931,28 +1025,13 @@ __global__ void bs_pairs_kernel(const double* __restrict__ x, const double* __re
     if (i >= n) return;
     const double xx[3] = {x[i * 3], x[i * 3 + 1], x[i * 3 + 2]};
     const double* yy = y + i * 6;
-    const double r0x = yy[3] - yy[0], r0y = yy[4] - yy[1], r0z = yy[5] - yy[2];
-    const double r0sq = r0x * r0x + r0y * r0y + r0z * r0z;
-    double acc[3] = {0.0, 0.0, 0.0};
-    if (kernel == FJ_KERNEL_EPSILON) {
-        Vtx64<FJ_KERNEL_EPSILON> a, b;
-        vtx64<FJ_KERNEL_EPSILON>(xx, yy[0], yy[1], yy[2], a);
-        vtx64<FJ_KERNEL_EPSILON>(xx, yy[3], yy[4], yy[5], b);
-        link64<FJ_KERNEL_EPSILON>(a, b, 1.0, r0x, r0y, r0z, kEps * r0sq * r0sq, rc2, acc);
-    } else if (kernel == FJ_KERNEL_CUTOFF) {
-        Vtx64<FJ_KERNEL_CUTOFF> a, b;
-        vtx64<FJ_KERNEL_CUTOFF>(xx, yy[0], yy[1], yy[2], a);
-        vtx64<FJ_KERNEL_CUTOFF>(xx, yy[3], yy[4], yy[5], b);
-        link64<FJ_KERNEL_CUTOFF>(a, b, 1.0, r0x, r0y, r0z, r0sq, rc2, acc);
-    } else {
-        Vtx64<FJ_KERNEL_PLAIN> a, b;
-        vtx64<FJ_KERNEL_PLAIN>(xx, yy[0], yy[1], yy[2], a);
-        vtx64<FJ_KERNEL_PLAIN>(xx, yy[3], yy[4], yy[5], b);
-        link64<FJ_KERNEL_PLAIN>(a, b, 1.0, r0x, r0y, r0z, r0sq, rc2, acc);
-    }
-    out[i * 3 + 0] = acc[0];
-    out[i * 3 + 1] = acc[1];
-    out[i * 3 + 2] = acc[2];
+    double acc[3];
+    if (kernel == FJ_KERNEL_EPSILON) segment64<FJ_KERNEL_EPSILON>(xx, yy, yy + 3, rc2, acc);
+    else if (kernel == FJ_KERNEL_CUTOFF) segment64<FJ_KERNEL_CUTOFF>(xx, yy, yy + 3, rc2, acc);
+    else segment64<FJ_KERNEL_PLAIN>(xx, yy, yy + 3, rc2, acc);
+    out[i * 3 + 0] = acc[0] * kInv4Pi;
+    out[i * 3 + 1] = acc[1] * kInv4Pi;
+    out[i * 3 + 2] = acc[2] * kInv4Pi;
 }
 
 int biot_savart_pairs(const double* x, const double* y, int64_t n, int kernel, double r_cut,

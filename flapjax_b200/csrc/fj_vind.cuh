@@ -67,16 +67,17 @@ struct PackArgs {
 int pack_stream64(const PackArgs& a, Elem64* out, cudaStream_t s);
 int pack_stream32(const PackArgs& a, Elem32* out, cudaStream_t s);
 
-// Target-set x stream sum with per-split partials.  `part` has n_split * n_targets * 3
-// doubles; `reduce_partials` then sums them in split order into `out` (+= when
+// Target-set x stream sum with per-piece partials.  `part` has n_split * n_sub * n_targets
+// * 3 doubles; `reduce_partials` then sums them in a fixed order into `out` (+= when
 // accumulate != 0).
 struct VindJob {
     const double* targets;  // (n_targets, 3)
     int64_t n_targets;
     const void* stream;     // Elem64* or Elem32*
     int64_t n_elem;
-    int n_split;
-    double* part;           // (n_split, n_targets, 3)
+    int n_split;            // cuts of the stream
+    int n_sub;              // pieces each split is cut into (one CTA and one partial each)
+    double* part;           // (n_split n_sub, n_targets, 3)
     int64_t n_links;        // filaments in the stream (for pair counting)
     double* out;            // (n_targets, 3) result of the reduction (batched launches)
     int accumulate;         // batched reduction: 1 adds the sum to out, 0 overwrites out
@@ -96,9 +97,9 @@ int vind_launch_jobs(const VindJob* d_jobs, const int64_t* d_cta0, int n_jobs, i
                      int tile = 0);
 int pack_jobs(const PackJob* d_jobs, int n_jobs, int64_t max_elem, int precision, cudaStream_t s);
 int reduce_jobs(const VindJob* d_jobs, int n_jobs, int64_t max_targets, cudaStream_t s);
-// CTAs of one sum (target tiles x splits), for building cta0; tile = targets per thread of
+// CTAs of one sum (target tiles x pieces), for building cta0; tile = targets per thread of
 // the FP32 sum (2 or 4; 0 = 2), ignored for FP64.
-int64_t vind_ctas(int64_t n_targets, int n_split, int precision, int tile = 0);
+int64_t vind_ctas(int64_t n_targets, int n_part, int precision, int tile = 0);
 
 // filaments of an (rows, cols) lattice: rows(cols+1) chordwise + (rows+1)cols spanwise
 inline int64_t lattice_links(int rows, int cols) {
@@ -107,7 +108,7 @@ inline int64_t lattice_links(int rows, int cols) {
 
 // tile: FP32 targets per thread (2 or 4); 0 takes the tuned table's choice for the shape.
 int vind_launch(const VindJob& job, int precision, int kernel, double r_cut, cudaStream_t s, int tile = 0);
-int reduce_partials(const double* part, int n_split, int64_t n_targets, double* out,
+int reduce_partials(const double* part, int n_part, int64_t n_targets, double* out,
                     int accumulate, double scale, cudaStream_t s);
 int choose_split(int64_t n_targets, int64_t n_elem, int precision);
 // FP32 targets per thread for a shape: 4 where the autotuner found the wide tile faster,
@@ -130,5 +131,9 @@ void tune_publish(const TuneTable* t);
 int tune_bucket_targets(int64_t n_targets);
 int tune_bucket_elem(int64_t n_elem);
 int split_bound(int64_t n_targets, int64_t n_elem_max, int precision);
+// Pieces per split for a sum whose partial buffer holds max_part partials, and the partials
+// any such sum may take (workspace sizing).
+int choose_sub(int64_t n_targets, int64_t n_elem, int n_split, int precision, int tile, int64_t max_part);
+int part_bound(int64_t n_targets, int64_t n_elem_max, int precision);
 
 }  // namespace fj
