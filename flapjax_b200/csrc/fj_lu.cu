@@ -13,11 +13,9 @@
 #include <climits>
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
-
-#include <cooperative_groups.h>
 
 #include "fj_lu.cuh"
+#include "fj_panel.cuh"
 #include "fj_tc.cuh"
 
 namespace fj {
@@ -660,10 +658,9 @@ int lu_inverse32(const float* lu, int n, const int32_t* piv, float* x, cudaStrea
 // ---------------------------------------------------------------------------------
 // Tensor-core factorisation and inverse (mixed path, n >= kTcMinN).
 //
-// lu_factor32_tc: the same partial-pivoting LU, blocked twice.  One thread-block cluster
-// factors each outer panel of 128 columns (lu_panel_cluster_kernel; the 16-column panels
-// above where the rows exceed one cluster, their U rows and updates confined to the outer
-// panel).  The columns to its right receive only the row swaps until the outer panel is
+// lu_factor32_tc: the same partial-pivoting LU, blocked twice.  One launch factors each
+// outer panel of 128 columns (panel_factor; the 16-column panels above where the rows
+// exceed one cluster, their U rows and updates confined to the outer panel).  The columns to its right receive only the row swaps until the outer panel is
 // done; then
 //   U12 = L11^-1 A12        (lu_trsm32_kernel: forward substitution, CUDA cores, in place)
 //   A22 -= L21 U12          (tensor cores, K = 128)
@@ -676,9 +673,7 @@ int lu_inverse32(const float* lu, int n, const int32_t* piv, float* x, cudaStrea
 constexpr int kTcBlk = 128;
 
 // tri: the 2 x nblk inverted diagonal blocks (L's, then U's), then the TMA products'
-// operand-split scratch, enough for the largest product (m, n <= nblk x 128, K = 128),
-// then the row-swap list of one outer panel (kSwapInts ints).
-constexpr int kSwapInts = 1 + 2 * 2 * kTcBlk;  // count, then (destination, source) row pairs
+// operand-split scratch, enough for the largest product (m, n <= nblk x 128, K = 128).
 
 static size_t tc_inv_floats(int n) {
     return (size_t)2 * ((n + kTcBlk - 1) / kTcBlk) * kTcBlk * kTcBlk;
@@ -690,471 +685,66 @@ static size_t tc_scratch_floats(int n) {
 }
 
 size_t tc_tri_floats(int n) {
-    return tc_inv_floats(n) + tc_scratch_floats(n) + (size_t)kSwapInts;
+    return tc_inv_floats(n) + tc_scratch_floats(n);
 }
 
-// ---------------------------------------------------------------------------------
-// One 128-column outer panel, (n - k) rows, factored by a single thread-block cluster
-// of 16-warp CTAs (up to 16 CTAs of 8-row warps where the device allows that cluster
-// size, else up to 8 CTAs of 16-row warps): getrf's partial pivoting and rank-1 updates
-// column by column, with the panel in registers.  Lanes are columns: lane L of a warp
-// holds columns L, L + 32, L + 64, L + 96 of the warp's RPW rows; CTA q holds panel rows
-// 16 RPW q .. in order over its warps.  The column loop runs in four groups of 32
-// (unrolled), so that a column's register is a compile-time index.  Per column j:
-//   a. every warp gathers column j of its rows (lane i takes row i from lane j % 32),
-//      finds the first maximum of |a(r, j)| over rows r >= j (keys are the magnitude's
-//      bits + 1, so one redux.sync orders them; NaN is never a candidate; the lowest
-//      lane, i.e. row, wins a tie) and copies the winning row into its candidate slot;
-//      the warp holding row j copies row j;
-//   b. one CTA barrier; four warps take the CTA's first maximum over its warps and push
-//      that row, its key, index and origin into every CTA's slot q (distributed shared
-//      memory stores); in CTA 0 four more warps push row j the same way;
-//   c. one cluster barrier;
-//   d. every warp reads the nc slot keys from its own shared memory and takes the first
-//      maximum (lowest CTA: the lowest row, getrf's tie rule; no candidate keeps the
-//      diagonal); rows j and p trade places (the pivot row and row j from the local
-//      slots); the rows below j are scaled as getrf scales them (by the reciprocal of the
-//      pivot when its magnitude is at least the smallest normal, else by division) and
-//      updated.
-// All slots alternate between two buffers with the column's parity: a buffer is written
-// again only after the next column's cluster barrier, which every CTA reaches after its
-// reads of it.  Lane i < RPW of a warp carries the original index of the warp's row i;
-// at the end the moved rows are listed as (destination, source) global row pairs, at
-// most 2 x 128, for lu_swap_rows_kernel.  Every thread passes every barrier (the loop
-// bounds are uniform over the cluster), so no wait depends on data.
-namespace cg = cooperative_groups;
-
-constexpr int kPcThreads = 512;
-constexpr int kPcWarps = kPcThreads / 32;
-constexpr int kPcMaxCtas = 16;
-
-// Panel element types.  A panel row is 512 bytes either way: 128 FP32 columns (the mixed
-// path's outer panel) or 64 FP64 columns (the FP64 path's); lane L holds columns L + 32 c,
-// c < NG.  The candidate key is the magnitude's bits + 1, ordered as the magnitudes; 0 = no
-// candidate (inactive, or NaN, which never wins a getrf pivot search).
-template <typename T>
-struct PanelType;
-template <>
-struct PanelType<float> {
-    static constexpr int NG = 4;
-    using Key = uint32_t;
-    __device__ static __forceinline__ Key key(float x) {
-        const float ax = fabsf(x);
-        return ax == ax ? __float_as_uint(ax) + 1u : 0u;
-    }
-    __device__ static __forceinline__ bool normal(float x) { return fabsf(x) >= 1.17549435e-38f; }  // FLT_MIN
-};
-template <>
-struct PanelType<double> {
-    static constexpr int NG = 2;
-    using Key = unsigned long long;
-    __device__ static __forceinline__ Key key(double x) {
-        const double ax = fabs(x);
-        return ax == ax ? (Key)__double_as_longlong(ax) + 1ull : 0ull;
-    }
-    __device__ static __forceinline__ bool normal(double x) { return fabs(x) >= 2.2250738585072014e-308; }  // DBL_MIN
+// The rows that an outer panel's pivots move (panel_factor), as a list of (destination,
+// source) global rows in shared memory: the panel's own rows, then the pivot rows below
+// them (a row named by several pivots is listed as often, each time with the same source).
+// Returns the list's length; the CTA's first 2 kb threads trace one row each.
+template <int KB>
+struct MoveList {
+    int p[KB], dst[2 * KB], src[2 * KB];
+    int count[2 * KB / 32];
 };
 
-// The warp's largest key (every lane gets it).
-__device__ __forceinline__ uint32_t warp_key_max(uint32_t k) { return __reduce_max_sync(0xffffffffu, k); }
-__device__ __forceinline__ unsigned long long warp_key_max(unsigned long long k) {
-    const uint32_t hi = (uint32_t)(k >> 32);
-    const uint32_t mhi = __reduce_max_sync(0xffffffffu, hi);
-    const uint32_t mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? (uint32_t)k : 0u);
-    return ((unsigned long long)mhi << 32) | mlo;
-}
-
-// Row `i` (a runtime index) of a thread's rows, as the NG columns this lane holds.
-template <typename T, int NG, int RPW>
-__device__ __forceinline__ void pick_row(const T (&v)[RPW][NG], int i, T (&out)[NG]) {
-#pragma unroll
-    for (int c = 0; c < NG; ++c) out[c] = v[0][c];
-#pragma unroll
-    for (int r = 1; r < RPW; ++r)
-        if (r == i) {
-#pragma unroll
-            for (int c = 0; c < NG; ++c) out[c] = v[r][c];
-        }
-}
-
-template <typename T, int NG, int RPW>
-__device__ __forceinline__ void put_row(T (&v)[RPW][NG], int i, const T (&in)[NG]) {
-#pragma unroll
-    for (int r = 0; r < RPW; ++r)
-        if (r == i) {
-#pragma unroll
-            for (int c = 0; c < NG; ++c) v[r][c] = in[c];
-        }
-}
-
-// Rank-1 update of the rows below j with multipliers column(j) * s (mul) or / s (div).
-template <typename T, int NG, int RPW, int G, bool kDiv>
-__device__ __forceinline__ void panel_update(T (&v)[RPW][NG], int rbase, int rows, int j, int jj, int lane, T s,
-                                             const T (&pc)[NG]) {
-#pragma unroll
-    for (int i = 0; i < RPW; ++i) {
-        const int r = rbase + i;
-        if (r > j && r < rows) {  // uniform over the warp
-            T l = kDiv ? v[i][G] / s : v[i][G] * s;
-            l = __shfl_sync(0xffffffffu, l, jj);  // lane jj's is the multiplier
-            if (lane == jj) v[i][G] = l;
-#pragma unroll
-            for (int c = G + 1; c < NG; ++c) v[i][c] -= l * pc[c];
-            if (lane > jj) v[i][G] -= l * pc[G];
-        }
-    }
-}
-
-// The panel's shared state (static shared memory of lu_panel_cluster_kernel).
-template <typename T>
-struct PanelShared {
-    static constexpr int KB = 32 * PanelType<T>::NG;
-    using Key = typename PanelType<T>::Key;
-    T cand[2][kPcWarps][KB];  // this CTA's warp candidates
-    Key wkey[2][kPcWarps];
-    int wrow[2][kPcWarps], wsrc[2][kPcWarps];
-    T rowj_loc[2][KB];                // row j, in CTA 0
-    T slot[2][kPcMaxCtas][KB];        // every CTA's candidate, pushed by that CTA
-    Key slot_key[2][kPcMaxCtas];
-    int slot_row[2][kPcMaxCtas], slot_src[2][kPcMaxCtas];
-    T rowj[2][KB];                    // row j, pushed by CTA 0
-    int rowj_src[2];
-    int rowj_src_loc[2];
-    int piv[KB];  // written out at the end: no global store inside the column loop
-    int info;
-    int wcnt[kPcWarps], cnt, off;
-};
-
-template <typename T, int RPW, int G>
-__device__ __forceinline__ void panel_columns(T (&v)[RPW][PanelType<T>::NG], int& orig, int k, int kb, int rows,
-                                              int q, int nc, int tid, cg::cluster_group& cl, PanelShared<T>& S) {
-    constexpr int NG = PanelType<T>::NG;
-    using Key = typename PanelType<T>::Key;
-    const int lane = tid & 31, warp = tid >> 5;
-    const int rbase = (q * kPcWarps + warp) * RPW;
-    const unsigned full = 0xffffffffu;
-    const int jend = min(kb, 32 * G + 32);
-#pragma unroll 1
-    for (int j = 32 * G; j < jend; ++j) {
-        const int jj = j & 31, par = j & 1;
-        // a. the warp's candidate: lane i < RPW takes column j of row i
-        T xj = T(0);
-#pragma unroll
-        for (int i = 0; i < RPW; ++i) {
-            const T t = __shfl_sync(full, v[i][G], jj);
-            if (lane == i) xj = t;
-        }
-        const int r = rbase + lane;
-        const Key key = (lane < RPW && r >= j && r < rows) ? PanelType<T>::key(xj) : Key(0);
-        const Key wmax = warp_key_max(key);
-        const unsigned hit = __ballot_sync(full, wmax != Key(0) && key == wmax);
-        const int bi = hit ? __ffs(hit) - 1 : 0;
-        const int bsrc = __shfl_sync(full, orig, bi);
-        if (hit != 0u) {
-            T row[NG];
-            pick_row<T, NG, RPW>(v, bi, row);
-#pragma unroll
-            for (int c = 0; c < NG; ++c) S.cand[par][warp][lane + 32 * c] = row[c];
-        }
-        if (lane == 0) {
-            S.wkey[par][warp] = wmax;
-            S.wrow[par][warp] = rbase + bi;
-            S.wsrc[par][warp] = bsrc;
-        }
-        const bool holds_j = j >= rbase && j < rbase + RPW;
-        const int ij = j - rbase;
-        const int jsrc = __shfl_sync(full, orig, holds_j ? ij : 0);
-        if (holds_j) {
-            T row[NG];
-            pick_row<T, NG, RPW>(v, ij, row);
-#pragma unroll
-            for (int c = 0; c < NG; ++c) S.rowj_loc[par][lane + 32 * c] = row[c];
-            if (lane == 0) S.rowj_src_loc[par] = jsrc;
-        }
-        __syncthreads();
-        // b. push: warps 0-3 the CTA's candidate, warps 4-7 of the CTA holding row j that
-        //    row; a row is 512 bytes, and thread t stores its float4 t % 32 into CTAs
-        //    t / 32 % 4, + 4, + 8, + 12
-        if (warp < 8) {
-            const int t = tid & 127, f = t & 31, c0 = t >> 5;
-            if (warp < 4) {
-                const Key kw = lane < kPcWarps ? S.wkey[par][lane] : Key(0);
-                const Key m = warp_key_max(kw);
-                const unsigned h = __ballot_sync(full, m != Key(0) && kw == m);
-                const int w = h ? __ffs(h) - 1 : 0;
-                const float4 val = reinterpret_cast<const float4*>(S.cand[par][w])[f];
-                const int prow_r = S.wrow[par][w], prow_s = S.wsrc[par][w];
-#pragma unroll
-                for (int u = 0; u < kPcMaxCtas / 4; ++u) {
-                    const int c = c0 + 4 * u;
-                    if (c < nc) {
-                        PanelShared<T>* R = cl.map_shared_rank(&S, c);
-                        reinterpret_cast<float4*>(R->slot[par][q])[f] = val;
-                        if (f == 0) {
-                            R->slot_key[par][q] = m;
-                            R->slot_row[par][q] = prow_r;
-                            R->slot_src[par][q] = prow_s;
-                        }
-                    }
-                }
-            } else if (q == j / (kPcWarps * RPW)) {
-                const float4 val = reinterpret_cast<const float4*>(S.rowj_loc[par])[f];
-                const int js = S.rowj_src_loc[par];
-#pragma unroll
-                for (int u = 0; u < kPcMaxCtas / 4; ++u) {
-                    const int c = c0 + 4 * u;
-                    if (c < nc) {
-                        PanelShared<T>* R = cl.map_shared_rank(&S, c);
-                        reinterpret_cast<float4*>(R->rowj[par])[f] = val;
-                        if (f == 0) R->rowj_src[par] = js;
-                    }
-                }
-            }
-        }
-        cl.sync();
-        // d. the cluster's pivot, from this CTA's own slots (every warp)
-        const Key ks = lane < nc ? S.slot_key[par][lane] : Key(0);
-        const Key m = warp_key_max(ks);
-        const unsigned h = __ballot_sync(full, m != Key(0) && ks == m);
-        const int o = h ? __ffs(h) - 1 : 0;  // the lowest CTA with the maximum
-        const T* prow = m != Key(0) ? S.slot[par][o] : S.rowj[par];
-        const int p = m != Key(0) ? S.slot_row[par][o] : j;  // no candidate: row j stays the pivot row
-        if (p != j) {
-            if (holds_j) {  // row j takes the pivot row
-                T row[NG];
-#pragma unroll
-                for (int c = 0; c < NG; ++c) row[c] = prow[lane + 32 * c];
-                put_row<T, NG, RPW>(v, ij, row);
-                if (lane == ij) orig = S.slot_src[par][o];
-            }
-            if (p >= rbase && p < rbase + RPW) {  // row p takes row j
-                T row[NG];
-#pragma unroll
-                for (int c = 0; c < NG; ++c) row[c] = S.rowj[par][lane + 32 * c];
-                put_row<T, NG, RPW>(v, p - rbase, row);
-                if (lane == p - rbase) orig = S.rowj_src[par];
-            }
-        }
-        const T pv = prow[j];
-        if (tid == 0) {
-            S.piv[j] = k + p;
-            if (pv == T(0) && S.info == 0) S.info = k + j + 1;
-        }
-        if (pv != T(0)) {
-            T pc[NG];
-#pragma unroll
-            for (int c = 0; c < NG; ++c) pc[c] = prow[lane + 32 * c];
-            if (PanelType<T>::normal(pv))  // getrf's sfmin test
-                panel_update<T, NG, RPW, G, false>(v, rbase, rows, j, jj, lane, T(1) / pv, pc);
-            else
-                panel_update<T, NG, RPW, G, true>(v, rbase, rows, j, jj, lane, pv, pc);
-        }
-    }
-}
-
-// swaps (may be null: the FP64 path derives the moves from the pivots instead) receives
-// the moved rows; run_flag (may be null): every CTA returns at once when *run_flag == 0.
-template <typename T, int RPW>
-__global__ void __launch_bounds__(kPcThreads, 1)
-    lu_panel_cluster_kernel(T* __restrict__ a, int n, int k, int kb, int32_t* __restrict__ piv,
-                            int* __restrict__ info, int* __restrict__ swaps, const int* __restrict__ run_flag) {
-    if (run_flag != nullptr && *run_flag == 0) return;  // the same for every CTA of the cluster
-    constexpr int NG = PanelType<T>::NG;
-    cg::cluster_group cl = cg::this_cluster();
-    __shared__ __align__(16) PanelShared<T> S;
-    const int q = (int)cl.block_rank(), nc = (int)cl.num_blocks();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int rows = n - k;
-    const int rbase = (q * kPcWarps + warp) * RPW;  // the warp's first panel row
-    const unsigned full = 0xffffffffu;
-    if (tid == 0) S.info = 0;
-
-    T v[RPW][NG];
-#pragma unroll
-    for (int i = 0; i < RPW; ++i) {
-        const bool has = rbase + i < rows;
-        const T* src = a + (int64_t)(k + (has ? rbase + i : 0)) * n + k + lane;
-#pragma unroll
-        for (int c = 0; c < NG; ++c) v[i][c] = (has && lane + 32 * c < kb) ? src[32 * c] : T(0);
-    }
-    int orig = rbase + lane;  // lanes < RPW: original panel row of the warp's row `lane`
-    cl.sync();                // every CTA of the cluster runs before any shared memory is written remotely
-
-    panel_columns<T, RPW, 0>(v, orig, k, kb, rows, q, nc, tid, cl, S);
-    panel_columns<T, RPW, 1>(v, orig, k, kb, rows, q, nc, tid, cl, S);
-    if constexpr (NG > 2) {
-        panel_columns<T, RPW, 2>(v, orig, k, kb, rows, q, nc, tid, cl, S);
-        panel_columns<T, RPW, 3>(v, orig, k, kb, rows, q, nc, tid, cl, S);
-    }
-#pragma unroll
-    for (int i = 0; i < RPW; ++i) {
-        if (rbase + i < rows) {
-            T* dst = a + (int64_t)(k + rbase + i) * n + k + lane;
-#pragma unroll
-            for (int c = 0; c < NG; ++c)
-                if (lane + 32 * c < kb) dst[32 * c] = v[i][c];
-        }
-    }
-    // the moved rows, in row order: (destination, source) global rows
-    const bool moved = lane < RPW && rbase + lane < rows && orig != rbase + lane;
-    const unsigned mb = __ballot_sync(full, moved);
-    if (lane == 0) S.wcnt[warp] = __popc(mb);
-    __syncthreads();  // also orders the last column's piv and info before their reads
-    if (q == 0) {
-        for (int j = tid; j < kb; j += kPcThreads) piv[k + j] = S.piv[j];
-        if (tid == 0 && S.info != 0 && *info == 0) *info = S.info;
-    }
-    if (warp == 0) {
-        const int cw = lane < kPcWarps ? S.wcnt[lane] : 0;
-        int inc = cw;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int y = __shfl_up_sync(full, inc, off);
-            if (lane >= off) inc += y;
-        }
-        if (lane < kPcWarps) S.wcnt[lane] = inc - cw;  // exclusive prefix over the warps
-        if (lane == 31) S.cnt = inc;
-    }
-    cl.sync();  // every CTA's count is published
-    if (tid == 0) {
-        int off = 0;
-        for (int c = 0; c < q; ++c) off += cl.map_shared_rank(&S, c)->cnt;
-        S.off = off;
-        if (q == nc - 1 && swaps != nullptr) swaps[0] = off + S.cnt;
+template <int KB>
+__device__ __forceinline__ int list_moves(const int32_t* __restrict__ piv, int k, int kb, MoveList<KB>& m) {
+    constexpr int NW = 2 * KB / 32;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if (t < kb) m.p[t] = piv[k + t] - k;
+    __syncthreads();
+    int pos = -1, src = -1;
+    unsigned moved = 0;
+    if (warp < NW) {
+        if (t < kb) pos = t;
+        else if (t >= KB && t < KB + kb && m.p[t - KB] >= kb) pos = m.p[t - KB];
+        src = swap_source(m.p, kb, pos);
+        moved = __ballot_sync(0xffffffffu, pos >= 0 && src != pos);
+        if (lane == 0) m.count[warp] = __popc(moved);
     }
     __syncthreads();
-    if (moved && swaps != nullptr) {
-        const int e = S.off + S.wcnt[warp] + __popc(mb & ((1u << lane) - 1u));
-        swaps[1 + 2 * e] = k + rbase + lane;
-        swaps[2 + 2 * e] = k + orig;
+    int total = 0, before = 0;
+    for (int w = 0; w < NW; ++w) {
+        if (w < warp) before += m.count[w];
+        total += m.count[w];
     }
-    cl.sync();  // no CTA exits while another may still read its shared memory
+    if (warp < NW && ((moved >> lane) & 1u)) {
+        const int o = before + __popc(moved & ((1u << lane) - 1u));
+        m.dst[o] = k + pos;
+        m.src[o] = k + src;
+    }
+    __syncthreads();
+    return total;
 }
 
-// The outer panel's row permutation (lu_panel_cluster_kernel's list) for every column
-// outside the panel: a CTA takes 32 columns, loads every listed source row's values into
-// shared memory, then stores them to their destinations (all loads before any store, so
-// the permutation's cycles need no order).
+// An outer panel's row moves for every column outside it: a CTA takes 32 columns, loads
+// every moved row's values into shared memory, then stores them to their destinations (all
+// loads before any store, so the permutation's cycles need no order).
 __global__ void __launch_bounds__(256) lu_swap_rows_kernel(float* __restrict__ a, int n, int k, int kb,
-                                                           const int* __restrict__ swaps) {
-    __shared__ int s_dst[2 * kTcBlk], s_src[2 * kTcBlk];
+                                                           const int32_t* __restrict__ piv) {
+    __shared__ MoveList<kTcBlk> m;
     __shared__ float tile[2 * kTcBlk][33];
-    const int cnt = min(swaps[0], 2 * kTcBlk);
-    for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
-        s_dst[e] = swaps[1 + 2 * e];
-        s_src[e] = swaps[2 + 2 * e];
-    }
-    __syncthreads();
+    const int cnt = list_moves<kTcBlk>(piv, k, kb, m);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int c = blockIdx.x * 32 + lane;
     const bool col = c < n && (c < k || c >= k + kb);
+#pragma unroll 8
     for (int e = warp; e < cnt; e += 8)
-        if (col) tile[e][lane] = a[(int64_t)s_src[e] * n + c];
+        if (col) tile[e][lane] = a[(int64_t)m.src[e] * n + c];
     __syncthreads();
     for (int e = warp; e < cnt; e += 8)
-        if (col) a[(int64_t)s_dst[e] * n + c] = tile[e][lane];
-}
-
-// The largest cluster of lu_panel_cluster_kernel<T> CTAs the device runs (16 where the
-// non-portable size is allowed, else 8; 0 if none), checked once per element type.
-template <typename T>
-static int cluster_panel_max() {
-    static std::once_flag once;
-    static int best = 0;
-    std::call_once(once, [] {
-        for (int size : {16, 8}) {
-            const void* fn = size == 16 ? (const void*)lu_panel_cluster_kernel<T, 8> : (const void*)lu_panel_cluster_kernel<T, 16>;
-            if (size == 16 && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-                cudaGetLastError();
-                continue;
-            }
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)size);
-            cfg.blockDim = dim3(kPcThreads);
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = (unsigned)size;
-            at[0].val.clusterDim.y = 1;
-            at[0].val.clusterDim.z = 1;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            int clusters = 0;
-            const cudaError_t e = size == 16 ? cudaOccupancyMaxActiveClusters(&clusters, lu_panel_cluster_kernel<T, 8>, &cfg)
-                                             : cudaOccupancyMaxActiveClusters(&clusters, lu_panel_cluster_kernel<T, 16>, &cfg);
-            cudaGetLastError();
-            if (e == cudaSuccess && clusters > 0) {
-                best = size;
-                break;
-            }
-        }
-    });
-    return best;
-}
-
-// Rows of the outer panel one cluster takes: 16 CTAs of 8-row warps, or 8 CTAs of
-// 16-row warps.
-template <typename T>
-static int cluster_panel_rows() {
-    const int m = cluster_panel_max<T>();
-    return m == 16 ? 16 * 8 * kPcWarps : m == 8 ? 8 * 16 * kPcWarps : 0;
-}
-
-// One cluster panel launch with RPW rows per warp: nc CTAs of kPcWarps warps.
-template <typename T, int RPW>
-static int launch_cluster_rpw(T* a, int n, int k, int kb, int32_t* piv, int* info, int* swaps, const int* run_flag,
-                              int nc, cudaStream_t s) {
-    if (nc > 8) {  // non-portable cluster size: allowed once per instantiation
-        static std::once_flag once;
-        static cudaError_t e = cudaSuccess;
-        std::call_once(once, [] {
-            e = cudaFuncSetAttribute((const void*)lu_panel_cluster_kernel<T, RPW>,
-                                     cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        });
-        FJ_CUDA(e);
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)nc);
-    cfg.blockDim = dim3(kPcThreads);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)nc;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    FJ_CUDA(cudaLaunchKernelEx(&cfg, lu_panel_cluster_kernel<T, RPW>, a, n, k, kb, piv, info, swaps, run_flag));
-    note_launch();
-    return FJ_OK;
-}
-
-// The cluster panel at column k (kb columns, n - k <= cluster_panel_rows<T>() rows), with
-// the fewest rows per warp (2, 4, 8 or 16) whose cluster the device runs: a column's
-// serial work in a warp grows with its rows (8-CTA clusters of 16-row warps factor the
-// 2048-row AIC 18 % slower than 16-CTA clusters of 8-row warps).
-template <typename T>
-static int launch_cluster_panel(T* a, int n, int k, int kb, int32_t* piv, int* info, int* swaps,
-                                const int* run_flag, cudaStream_t s) {
-    const int max_nc = cluster_panel_max<T>();
-    const int rows = n - k;
-    int rpw = 2;
-    while (rpw < 16 && (rows + kPcWarps * rpw - 1) / (kPcWarps * rpw) > max_nc) rpw *= 2;
-    const int nc = (rows + kPcWarps * rpw - 1) / (kPcWarps * rpw);
-    if (nc > max_nc || nc < 1) return fail(FJ_ERR_UNSUPPORTED, "cluster panel: %d rows", rows);
-    switch (rpw) {
-        case 2: return launch_cluster_rpw<T, 2>(a, n, k, kb, piv, info, swaps, run_flag, nc, s);
-        case 4: return launch_cluster_rpw<T, 4>(a, n, k, kb, piv, info, swaps, run_flag, nc, s);
-        case 8: return launch_cluster_rpw<T, 8>(a, n, k, kb, piv, info, swaps, run_flag, nc, s);
-        default: return launch_cluster_rpw<T, 16>(a, n, k, kb, piv, info, swaps, run_flag, nc, s);
-    }
-}
-
-static int launch_panel_cluster(float* a, int n, int k, int kb, int32_t* piv, int* info, int* swaps,
-                                cudaStream_t s) {
-    FJ_TRY(launch_cluster_panel<float>(a, n, k, kb, piv, info, swaps, nullptr, s));
-    lu_swap_rows_kernel<<<(unsigned)((n + 31) / 32), 256, 0, s>>>(a, n, k, kb, swaps);
-    note_launch();
-    return FJ_OK;
+        if (col) a[(int64_t)m.dst[e] * n + c] = tile[e][lane];
 }
 
 // U12 = L11^-1 A12 for the mixed factorisation's outer panel at column k (kb <= 128
@@ -1232,12 +822,15 @@ static int lu_factor32_tc_impl(float* a, int n, int32_t* piv, int* d_info, int* 
     FJ_TRY(allow_dynamic_smem((const void*)lu_panel_reg_kernel<float, NB, 2>, smem));
     FJ_TRY(allow_dynamic_smem((const void*)lu_trsm32_kernel, kTrsm32Smem));
     FJ_CUDA(cudaMemsetAsync(d_info, 0, sizeof(int), s));
-    int* swaps = reinterpret_cast<int*>(tri_l + tc_inv_floats(n) + tc_scratch_floats(n));
-    const int cluster_rows = cluster_panel_rows<float>();
+    const int panel_rows = panel_max_rows<float>();
     for (int k = 0; k < n; k += kTcBlk) {
         const int kb = min(kTcBlk, n - k), ke = k + kb;
-        if (n - k <= cluster_rows) {
-            FJ_TRY(launch_panel_cluster(a, n, k, kb, piv, d_info, swaps, s));
+        if (n - k <= panel_rows) {
+            FJ_TRY(panel_factor<float>(a, n, k, kb, piv, d_info, nullptr, s));
+            if (n > kb) {
+                lu_swap_rows_kernel<<<(unsigned)((n + 31) / 32), 256, 0, s>>>(a, n, k, kb, piv);
+                note_launch();
+            }
         } else {
           for (int j = k; j < ke; j += NB) {
             const int nb = min(NB, n - j);
@@ -1332,9 +925,9 @@ int lu_inverse32_tc(const float* lu, int n, const int32_t* piv, float* x, float*
 
 // ---------------------------------------------------------------------------------
 // FP64 factorisation (the plain path's getrf), blocked twice.  Outer panels of kDB = 64
-// columns; where a panel's rows fit one cluster (n - k <= cluster_panel_rows<double>())
-// one lu_panel_cluster_kernel<double> launch factors it, else 2- to 8-column panels do,
-// with their U rows and updates confined to the outer panel.  Then
+// columns; where a panel's rows fit one launch (n - k <= panel_max_rows<double>())
+// panel_factor factors it, else 2- to 8-column panels do, with their U rows and updates
+// confined to the outer panel.  Then
 //   lu_swap_trsm64_kernel: the outer panel's row swaps for every column outside it, and
 //                          U12 = L11^-1 A12 for the columns to its right;
 //   lu_gemm64_kernel:      A22 -= L21 U12 (K = 64, FP64 FMA).
@@ -1342,13 +935,14 @@ int lu_inverse32_tc(const float* lu, int n, const int32_t* piv, float* x, float*
 // matrix is updated once per 64 columns instead of once per column, so the factors
 // differ from a column-by-column getrf only by rounding.
 constexpr int kDB = 64;
+static_assert(kDB == kPanelCols<double> && kTcBlk == kPanelCols<float>, "the outer panels are panel_factor's");
 
-// The composed row moves of the outer panel at column k, from its kb pivots applied in
-// order (getrf's laswp): map[i] = the panel row whose values end at panel row i.  A move
-// lands on a row < k + kb, or on a pivot row at or below k + kb.  For the columns outside
-// the panel each CTA (32 columns, one per lane) loads every moved value before it stores
-// any.  Then, for the CTA's columns right of the panel, the kb x kb unit-lower L11 solves
-// its rows k .. k + kb: warp w (of 16) takes columns 2w and 2w + 1, lane l rows l and l + 32.
+// The outer panel's row moves for 32 columns per CTA, one per lane: the panel's own kb rows
+// come from the rows whose values end there (swap_source), the rows below it that move are
+// listed and loaded beside them, and every load precedes every store.  Then, for the CTA's
+// columns right of the panel, the kb x kb unit-lower L11 solves the panel's rows: warp w (of
+// 16) takes columns 2w and 2w + 1 side by side (their chains of shuffles overlap), lane l
+// rows l and l + 32.  Latency-bound: one round trip to memory, then 64 substitution steps.
 constexpr int kSwapTrsm64Warps = 16;
 
 __global__ void __launch_bounds__(32 * kSwapTrsm64Warps)
@@ -1356,92 +950,93 @@ __global__ void __launch_bounds__(32 * kSwapTrsm64Warps)
                           int do_swaps, const int* __restrict__ run_flag) {
     if (run_flag != nullptr && *run_flag == 0) return;
     extern __shared__ __align__(16) unsigned char sm64[];
-    double* tile = reinterpret_cast<double*>(sm64);            // [2 kDB][32] moved values; then x [kDB][33]
-    double* ls = tile + 2 * kDB * 33;                          // [kDB][kDB + 1] L11
-    int* map = reinterpret_cast<int*>(ls + kDB * (kDB + 1));  // [n - k]
-    __shared__ int s_dst[2 * kDB], s_src[2 * kDB];
-    __shared__ int s_cnt;
+    double* xs = reinterpret_cast<double*>(sm64);  // [kDB][33]
+    double* ls = xs + kDB * 33;                    // [kDB][kDB + 1] L11
+    __shared__ int p[kDB], src[kDB], down_dst[kDB], down_src[kDB];
     const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int rows = n - k, c0 = blockIdx.x * 32, c = c0 + lane;
-    if (do_swaps) {
-        for (int i = threadIdx.x; i < rows; i += blockDim.x) map[i] = i;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int j = 0; j < kb; ++j) {
-                const int p = piv[k + j] - k;
-                if (p != j && p > j && p < rows) {
-                    const int t = map[j];
-                    map[j] = map[p];
-                    map[p] = t;
-                }
-            }
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int c0 = blockIdx.x * 32, c = c0 + lane;
+    const bool solve = c0 + 31 >= k + kb && kb > 1;  // a column right of the panel (uniform over the CTA)
+    if (t < kb) p[t] = do_swaps ? piv[k + t] - k : t;
+    if (solve) {
+#pragma unroll
+        for (int idx = t; idx < kDB * kDB; idx += 32 * kSwapTrsm64Warps) {
+            const int r = idx / kDB, j = idx % kDB;
+            ls[r * (kDB + 1) + j] = (r < kb && j < r) ? a[(int64_t)(k + r) * n + k + j] : 0.0;
         }
-        __syncthreads();
-        if (warp == 0) {  // the moves, listed: rows [0, kb), then the pivot rows at or below kb
-            int base = 0;
-            for (int e0 = 0; e0 < 2 * kb; e0 += 32) {
-                const int e = e0 + lane;
-                int pos = -1;
-                if (e < kb) {
-                    pos = e;
-                } else if (e < 2 * kb) {
-                    const int p = piv[k + e - kb] - k;
-                    if (p >= kb && p < rows) pos = p;
-                }
-                const bool mv = pos >= 0 && map[pos] != pos;
-                const unsigned m = __ballot_sync(full, mv);
-                if (mv) {
-                    const int o = base + __popc(m & ((1u << lane) - 1u));
-                    s_dst[o] = k + pos;
-                    s_src[o] = k + map[pos];
-                }
-                base += __popc(m);
-            }
-            if (lane == 0) s_cnt = base;
-        }
-        __syncthreads();
-        const int cnt = s_cnt;
-        const bool col = c < n && (c < k || c >= k + kb);
-        for (int e = warp; e < cnt; e += kSwapTrsm64Warps)
-            if (col) tile[e * 32 + lane] = a[(int64_t)s_src[e] * n + c];
-        __syncthreads();
-        for (int e = warp; e < cnt; e += kSwapTrsm64Warps)
-            if (col) a[(int64_t)s_dst[e] * n + c] = tile[e * 32 + lane];
-        __syncthreads();  // the CTA's stores are seen by its loads below
-    }
-    if (c0 + 31 < k + kb || kb < 2) return;  // no column right of the panel (uniform over the CTA)
-    for (int idx = threadIdx.x; idx < kDB * kDB; idx += blockDim.x) {
-        const int r = idx / kDB, j = idx % kDB;
-        ls[r * (kDB + 1) + j] = (r < kb && j < r) ? a[(int64_t)(k + r) * n + k + j] : 0.0;
-    }
-    double* xs = tile;
-    for (int idx = threadIdx.x; idx < kDB * 32; idx += blockDim.x) {
-        const int r = idx >> 5, cc = idx & 31, cg_ = c0 + cc;
-        xs[r * 33 + cc] = (r < kb && cg_ >= k + kb && cg_ < n) ? a[(int64_t)(k + r) * n + cg_] : 0.0;
     }
     __syncthreads();
-#pragma unroll 1
-    for (int t = 0; t < 2; ++t) {
-        const int cc = warp * 2 + t;
-        double x0 = xs[lane * 33 + cc], x1 = xs[(lane + 32) * 33 + cc];
+    if (t < kb) {
+        src[t] = do_swaps ? swap_source(p, kb, t) : t;
+    } else if (t >= kDB && t < kDB + kb) {
+        const int r = p[t - kDB];  // a row below the panel takes the values that end there
+        down_dst[t - kDB] = r >= kb ? r : -1;
+        down_src[t - kDB] = r >= kb ? swap_source(p, kb, r) : 0;
+    }
+    __syncthreads();
+    const bool col = c < n && (c < k || c >= k + kb);
+    double own[kDB / kSwapTrsm64Warps], down[kDB / kSwapTrsm64Warps];
+#pragma unroll
+    for (int i = 0; i < kDB / kSwapTrsm64Warps; ++i) {
+        const int r = warp + i * kSwapTrsm64Warps;
+        own[i] = r < kb && col ? a[(int64_t)(k + src[r]) * n + c] : 0.0;
+        down[i] = r < kb && col && down_dst[r] >= 0 ? a[(int64_t)(k + down_src[r]) * n + c] : 0.0;
+    }
+    __syncthreads();  // the CTA has read what it is about to write
+#pragma unroll
+    for (int i = 0; i < kDB / kSwapTrsm64Warps; ++i) {
+        const int r = warp + i * kSwapTrsm64Warps;
+        if (r < kb && col && down_dst[r] >= 0) a[(int64_t)(k + down_dst[r]) * n + c] = down[i];
+        if (solve) xs[r * 33 + lane] = own[i];
+        else if (r < kb && col) a[(int64_t)(k + r) * n + c] = own[i];
+    }
+    if (!solve) return;
+    __syncthreads();
+    double x0[2], x1[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        x0[h] = xs[lane * 33 + 2 * warp + h];
+        x1[h] = xs[(lane + 32) * 33 + 2 * warp + h];
+    }
+    const bool right0 = c0 + 2 * warp >= k + kb, right1 = c0 + 2 * warp + 1 >= k + kb;
+    if (right0 || right1) {  // (columns left of the panel only move)
+        const double *l0 = ls + lane * (kDB + 1), *l1 = ls + (lane + 32) * (kDB + 1);
+        double y0[2] = {x0[0], x0[1]}, y1[2] = {x1[0], x1[1]};
 #pragma unroll 4
-        for (int j = 0; j < kb - 1; ++j) {
-            const double xj = __shfl_sync(full, j < 32 ? x0 : x1, j & 31);
-            if (lane > j) x0 -= ls[lane * (kDB + 1) + j] * xj;
-            x1 -= ls[(lane + 32) * (kDB + 1) + j] * xj;  // rows >= kb: zero multipliers
+        for (int j = 0; j < min(kb - 1, 32); ++j) {
+            const double m0 = l0[j], m1 = l1[j];  // rows >= kb: zero multipliers
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const double xj = __shfl_sync(full, y0[h], j);
+                if (lane > j) y0[h] -= m0 * xj;
+                y1[h] -= m1 * xj;
+            }
         }
-        xs[lane * 33 + cc] = x0;
-        xs[(lane + 32) * 33 + cc] = x1;
+#pragma unroll 4
+        for (int j = 32; j < kb - 1; ++j) {
+            const double m1 = l1[j];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const double xj = __shfl_sync(full, y1[h], j - 32);
+                y1[h] -= m1 * xj;
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (h == 0 ? right0 : right1) {
+                xs[lane * 33 + 2 * warp + h] = y0[h];
+                xs[(lane + 32) * 33 + 2 * warp + h] = y1[h];
+            }
     }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < kDB * 32; idx += blockDim.x) {
-        const int r = idx >> 5, cc = idx & 31, cg_ = c0 + cc;
-        if (r >= 1 && r < kb && cg_ >= k + kb && cg_ < n) a[(int64_t)(k + r) * n + cg_] = xs[r * 33 + cc];
+#pragma unroll
+    for (int idx = t; idx < kDB * 32; idx += 32 * kSwapTrsm64Warps) {
+        const int r = idx >> 5, cc = idx & 31, g = c0 + cc;
+        if (r < kb && g < n && (g < k || g >= k + kb)) a[(int64_t)(k + r) * n + g] = xs[r * 33 + cc];
     }
 }
 
-constexpr size_t kSwapTrsm64Fixed = (size_t)(2 * kDB * 33 + kDB * (kDB + 1)) * sizeof(double);
+constexpr size_t kSwapTrsm64Smem = (size_t)(kDB * 33 + kDB * (kDB + 1)) * sizeof(double);
 
 // A22 -= L21 U12 with K = kDB, on one 64 x 64 tile of the trailing matrix per CTA: the
 // CTA's 64 rows of L21 and 64 columns of U12 come into shared memory (cp.async, zero past
@@ -1533,18 +1128,17 @@ int lu_factor64(double* a, int n, int32_t* piv, int* d_info, cudaStream_t s, con
     int nb_narrow = 0;
     for (int nb : {8, 4, 2})
         if (nb_narrow == 0 && panel_fits<double>(n, nb)) nb_narrow = nb;
-    const int cluster_rows = cluster_panel_rows<double>();
-    if (nb_narrow == 0 && n > cluster_rows)
+    const int panel_rows = panel_max_rows<double>();
+    if (nb_narrow == 0 && n > panel_rows)
         return fail(FJ_ERR_UNSUPPORTED, "lu_factor: n=%d too large for the shared-memory panel", n);
-    const size_t st_smem = kSwapTrsm64Fixed + (size_t)n * sizeof(int);
-    FJ_TRY(allow_dynamic_smem((const void*)lu_swap_trsm64_kernel, st_smem));
+    FJ_TRY(allow_dynamic_smem((const void*)lu_swap_trsm64_kernel, kSwapTrsm64Smem));
     FJ_TRY(allow_dynamic_smem((const void*)lu_gemm64_kernel, kGemm64Smem));
     FJ_CUDA(cudaMemsetAsync(d_info, 0, sizeof(int), s));
     for (int k = 0; k < n; k += kDB) {
         const int kb = min(kDB, n - k), ke = k + kb;
-        const bool cluster = n - k <= cluster_rows;
-        if (cluster) {
-            FJ_TRY(launch_cluster_panel<double>(a, n, k, kb, piv, d_info, nullptr, run_flag, s));
+        const bool whole = n - k <= panel_rows;
+        if (whole) {
+            FJ_TRY(panel_factor<double>(a, n, k, kb, piv, d_info, run_flag, s));
         } else if (nb_narrow == 8) {
             FJ_TRY(lu_outer_panel_narrow64<8>(a, n, k, ke, piv, d_info, run_flag, s));
         } else if (nb_narrow == 4) {
@@ -1553,8 +1147,8 @@ int lu_factor64(double* a, int n, int32_t* piv, int* d_info, cudaStream_t s, con
             FJ_TRY(lu_outer_panel_narrow64<2>(a, n, k, ke, piv, d_info, run_flag, s));
         }
         if (n > kb) {
-            lu_swap_trsm64_kernel<<<(unsigned)((n + 31) / 32), 32 * kSwapTrsm64Warps, st_smem, s>>>(
-                a, n, k, kb, piv, cluster ? 1 : 0, run_flag);
+            lu_swap_trsm64_kernel<<<(unsigned)((n + 31) / 32), 32 * kSwapTrsm64Warps, kSwapTrsm64Smem, s>>>(
+                a, n, k, kb, piv, whole ? 1 : 0, run_flag);
             note_launch();
         }
         const int rest = n - ke;

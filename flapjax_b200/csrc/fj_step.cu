@@ -1794,7 +1794,7 @@ static int check_buffers(const Plan& p, const fj_case_buffers* B, bool dynamic) 
 }
 
 // Status words of a case-level call: flags[0] the LU info of the last factorisation
-// (first zero pivot + 1), flags[2] the lowest slot with a non-finite total force,
+// (first zero pivot + 1; the order + 1 where a panel's bounded wait expired), flags[2] the lowest slot with a non-finite total force,
 // flags[3] set when a bounded wait of the tensor-core factorisation expired, flags[4] set
 // when a replayed step graph found its slot counter out of range.
 static constexpr int kNoSlot = 0x7f7f7f7f;  // the byte pattern 0x7f repeated
@@ -1810,6 +1810,7 @@ static int read_status(const Plan& p, cudaStream_t s) {
     FJ_CUDA(cudaStreamSynchronize(s));
     if (w[4] != 0) return fail(FJ_ERR_CUDA, "a replayed step graph found its slot counter out of range");
     if (w[3] != 0) return fail(FJ_ERR_TIMEOUT, "a tensor-core wait of the AIC factorisation expired");
+    if (w[0] > p.nb) return fail(FJ_ERR_TIMEOUT, "a wait of the AIC factorisation's panels expired");
     if (w[2] != kNoSlot) return fail(FJ_ERR_NONFINITE, "non-finite forces at time slot %d", w[2]);
     if (w[0] != 0) return fail(FJ_ERR_SINGULAR, "zero pivot in column %d of the AIC factorisation", w[0] - 1);
     return FJ_OK;
