@@ -21,8 +21,8 @@
 #include <cstring>
 #include <vector>
 
-#include "fj_lu.cuh"
 #include "fj_bsgrad.cuh"
+#include "fj_trsv.cuh"
 #include "fj_vind.cuh"
 
 namespace fj {
@@ -203,112 +203,6 @@ __global__ void unpack_gamma_kernel(UnpackArgs u, const double* __restrict__ el,
     u.gamma_bar[li][r] += (double)L.sign * gbar;
 }
 
-// ------------------------------------------------------------------------------------
-// getrs with A^T: A = P^T L U  =>  U^T L^T (P x) = b
-// ------------------------------------------------------------------------------------
-constexpr int kTBlk = 64;
-
-// The diagonal block [i0, i0 + bw) of the factors comes into shared memory as it lies in
-// memory (row-major, every element's cp.async in flight at once); one warp substitutes,
-// lane l holding x of rows l and l + 32 in registers and x_j reaching every lane by a
-// shuffle, reading the block transposed.  Per row the operations are those of the
-// column-by-column transposed substitution, in its order.
-__global__ void __launch_bounds__(kTBlk) trsv_t_diag_kernel(const double* __restrict__ lu, int n, int i0, int bw,
-                                                            bool upper_of_lt, double* __restrict__ x) {
-    // upper_of_lt == false: solve with U^T (lower, diagonal U[j][j]) forward
-    // upper_of_lt == true:  solve with L^T (upper, unit diagonal) backward
-    static_assert(kTBlk == 64, "two rows per lane");
-    __shared__ __align__(16) double blk[kTBlk][kTBlk + 1];  // blk[j][r] = lu[i0 + j][i0 + r]
-    for (int idx = threadIdx.x; idx < bw * bw; idx += blockDim.x) {
-        const int j = idx / bw, r = idx % bw;
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(&blk[j][r])),
-                     "l"(lu + (int64_t)(i0 + j) * n + i0 + r)
-                     : "memory");
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-    if (threadIdx.x >= 32) return;
-    const int lane = threadIdx.x;
-    const unsigned full = 0xffffffffu;
-    double v0 = lane < bw ? x[i0 + lane] : 0.0;
-    double v1 = lane + 32 < bw ? x[i0 + lane + 32] : 0.0;
-    if (!upper_of_lt) {
-#pragma unroll 1
-        for (int j = 0; j < bw; ++j) {
-            const bool hi = j >= 32;
-            if (lane == (j & 31)) {
-                if (hi) v1 = v1 / blk[j][j];
-                else v0 = v0 / blk[j][j];
-            }
-            const double xj = __shfl_sync(full, hi ? v1 : v0, j & 31);
-            if (lane > j && lane < bw) v0 -= blk[j][lane] * xj;
-            if (lane + 32 > j && lane + 32 < bw) v1 -= blk[j][lane + 32] * xj;
-        }
-    } else {
-#pragma unroll 1
-        for (int j = bw - 1; j >= 0; --j) {
-            const double xj = __shfl_sync(full, j >= 32 ? v1 : v0, j & 31);
-            if (lane < j) v0 -= blk[j][lane] * xj;
-            if (lane + 32 < j) v1 -= blk[j][lane + 32] * xj;
-        }
-    }
-    if (lane < bw) x[i0 + lane] = v0;
-    if (lane + 32 < bw) x[i0 + lane + 32] = v1;
-}
-
-// x[i] -= sum_{j in [j0, j0+bw)} lu[j][i] x[j] for i in [r0, r1)
-__global__ void trsv_t_update_kernel(const double* __restrict__ lu, int n, int j0, int bw, int r0, int r1,
-                                     double* __restrict__ x) {
-    const int i = r0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= r1) return;
-    double acc = 0.0;
-    for (int j = 0; j < bw; ++j) acc += lu[(int64_t)(j0 + j) * n + i] * x[j0 + j];
-    x[i] -= acc;
-}
-
-__global__ void __launch_bounds__(1024) unpermute_kernel(const int32_t* __restrict__ piv, int n,
-                                                         const double* __restrict__ w, double* __restrict__ x) {
-    extern __shared__ int perm[];
-    for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = i;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < n; ++i) {
-            const int p = piv[i];
-            if (p != i) {
-                const int t = perm[i];
-                perm[i] = perm[p];
-                perm[p] = t;
-            }
-        }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) x[perm[i]] = w[i];
-}
-
-int lu_solve_t64(const double* lu, int n, const int32_t* piv, double* b, double* work, cudaStream_t s) {
-    if (n <= 0) return fail(FJ_ERR_SHAPE, "lu_solve_t: n=%d", n);
-    if ((size_t)n * sizeof(int) > 220 * 1024) return fail(FJ_ERR_UNSUPPORTED, "lu_solve_t: n=%d too large", n);
-    FJ_CUDA(cudaMemcpyAsync(work, b, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    for (int i0 = 0; i0 < n; i0 += kTBlk) {  // U^T z = b, forward
-        const int bw = min(kTBlk, n - i0);
-        trsv_t_diag_kernel<<<1, kTBlk, 0, s>>>(lu, n, i0, bw, false, work); note_launch();
-        if (i0 + bw < n) {
-            trsv_t_update_kernel<<<(n - i0 - bw + 127) / 128, 128, 0, s>>>(lu, n, i0, bw, i0 + bw, n, work); note_launch();
-        }
-    }
-    for (int i0 = ((n - 1) / kTBlk) * kTBlk; i0 >= 0; i0 -= kTBlk) {  // L^T w = z, backward
-        const int bw = min(kTBlk, n - i0);
-        trsv_t_diag_kernel<<<1, kTBlk, 0, s>>>(lu, n, i0, bw, true, work); note_launch();
-        if (i0 > 0) {
-            trsv_t_update_kernel<<<(i0 + 127) / 128, 128, 0, s>>>(lu, n, i0, bw, 0, i0, work); note_launch();
-        }
-    }
-    FJ_TRY(allow_dynamic_smem((const void*)unpermute_kernel, (size_t)(n * sizeof(int))));
-    unpermute_kernel<<<1, 1024, n * sizeof(int), s>>>(piv, n, work, b); note_launch();
-    FJ_LAUNCH_CHECK("lu_solve_t64");
-    return FJ_OK;
-}
-
 static int64_t vjp_elems(const int* rows, const int* cols, int n_lattices, int img) {
     int64_t n = 0;
     for (int i = 0; i < n_lattices; ++i) n += img * stream_len(rows[i], cols[i]);
@@ -439,7 +333,9 @@ int fj_vind_vjp(const double* d_targets, int64_t n_targets, const double* const*
 int fj_lu_solve_t(const double* d_lu, int n, const int32_t* d_piv, double* d_b, void* d_ws, size_t ws_bytes,
                   fj_stream_t stream) {
     if (ws_bytes < 256 + (size_t)n * sizeof(double)) return fail(FJ_ERR_NOMEM, "lu_solve_t workspace too small");
-    return lu_solve_t64(d_lu, n, d_piv, d_b, (double*)((char*)d_ws + 256), (cudaStream_t)stream);
+    if (n <= 0) return fail(FJ_ERR_SHAPE, "lu_solve_t: n=%d", n);
+    // A = P^T L U  =>  U^T L^T (P x) = b
+    return lu_substitute64(d_lu, n, d_piv, d_b, (double*)((char*)d_ws + 256), true, (cudaStream_t)stream);
 }
 
 }  // extern "C"

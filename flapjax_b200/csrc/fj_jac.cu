@@ -25,6 +25,7 @@
 
 #include "fj_bs.cuh"
 #include "fj_bsgrad.cuh"
+#include "fj_trsv.cuh"
 #include "fj_vind.cuh"
 
 namespace fj {
@@ -199,17 +200,12 @@ __global__ void __launch_bounds__(kJacBlock) vertex_jacobian_kernel(const double
 }
 
 // perm = the getrf row swaps of piv applied in order to the identity
-__global__ void perm_from_piv_kernel(const int32_t* __restrict__ piv, int n, int32_t* __restrict__ perm) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    for (int i = 0; i < n; ++i) perm[i] = i;
-    for (int i = 0; i < n; ++i) {
-        const int p = piv[i];
-        if (p != i && p >= 0 && p < n) {
-            const int32_t t = perm[i];
-            perm[i] = perm[p];
-            perm[p] = t;
-        }
-    }
+__global__ void __launch_bounds__(1024) perm_from_piv_kernel(const int32_t* __restrict__ piv, int n,
+                                                             int32_t* __restrict__ perm) {
+    extern __shared__ int perm_sm[];
+    __shared__ PermScratch S;
+    build_perm(piv, n, perm_sm, S);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = perm_sm[i];
 }
 
 // Blocked substitution for many right-hand sides.  CTA = 256 threads on a tile of 32
@@ -447,7 +443,8 @@ int fj_lu_solve_many(const double* d_lu, int n, const int32_t* d_piv, double* d_
     char* base = (char*)(((uintptr_t)d_ws + 255) / 256 * 256);
     int32_t* perm = (int32_t*)base;
     double* w = (double*)(base + ((size_t)n * sizeof(int32_t) + 255) / 256 * 256);
-    perm_from_piv_kernel<<<1, 32, 0, s>>>(d_piv, n, perm);
+    FJ_TRY(allow_dynamic_smem((const void*)perm_from_piv_kernel, (size_t)n * sizeof(int)));
+    perm_from_piv_kernel<<<1, 1024, (size_t)n * sizeof(int), s>>>(d_piv, n, perm);
     lu_solve_many_kernel<<<(unsigned)((nrhs + kSolveCols - 1) / kSolveCols), kSolveThreads, 0, s>>>(d_lu, n, perm, d_b,
                                                                                              nrhs, ldb, w);
     note_launch(2);

@@ -6,7 +6,6 @@
 //      block arg-max with LAPACK's first-maximum tie rule, row swap, scale, rank-1);
 //   2. the panel's row swaps are applied to the other columns, and U12 = L11^-1 A12;
 //   3. the trailing matrix is updated, A22 -= L21 U12.
-// lu_solve64: getrs (pivots, unit-lower forward, upper backward substitution) in one CTA.
 // lu_inverse32 + refine_solve: the mixed-precision solve.  FP32 factors give an FP32
 // explicit inverse X once per factorisation; every solve is then GEMVs over all SMs:
 // x = X b, r = b - A x in FP64, x += X r.
@@ -17,6 +16,7 @@
 #include "fj_lu.cuh"
 #include "fj_panel.cuh"
 #include "fj_tc.cuh"
+#include "fj_trsv.cuh"
 
 namespace fj {
 
@@ -429,142 +429,14 @@ static bool panel_fits(int n, int nb) {
     return (size_t)n * (nb + 1) * sizeof(T) <= (size_t)220 * 1024;
 }
 
+int lu_solve64(const double* lu, int n, const int32_t* piv, double* b, double* work, cudaStream_t s) {
+    if (n <= 0) return fail(FJ_ERR_SHAPE, "lu_solve: n=%d", n);
+    return lu_substitute64(lu, n, piv, b, work, false, s);
+}
+
 int lu_factor32(float* a, int n, int32_t* piv, int* d_info, cudaStream_t s) {
     if (panel_fits<float>(n, 16)) return lu_factor_impl<float, 16>(a, n, piv, d_info, s, nullptr);
     return lu_factor_impl<float, 8>(a, n, piv, d_info, s, nullptr);
-}
-
-// ---------------------------------------------------------------------------------
-// getrs: x = P b, then blocked substitution.  Per block of kTrsvBlk rows one CTA solves
-// the diagonal block in shared memory and a grid of warps (one per remaining row) applies
-// the block's contribution to the rows still to be solved.
-constexpr int kTrsvBlk = 128;
-
-// x[i] = b[perm[i]], perm from the getrf row swaps applied in order to the identity.
-__global__ void __launch_bounds__(1024) permute_kernel(const int32_t* __restrict__ piv, int n,
-                                                       const double* __restrict__ b, double* __restrict__ x) {
-    extern __shared__ int perm[];  // n permutation entries, then n pivots
-    int* sp = perm + n;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        perm[i] = i;
-        sp[i] = piv[i];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {  // the swaps compose in order; from shared memory only
-        for (int i = 0; i < n; ++i) {
-            const int p = sp[i];
-            if (p != i) {
-                const int t = perm[i];
-                perm[i] = perm[p];
-                perm[p] = t;
-            }
-        }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) x[i] = b[perm[i]];
-}
-
-// Solve the diagonal block [i0, i0+bw) of L (unit lower, upper = false) or U (upper = true)
-// in place on x.  The block comes into shared memory with every element's cp.async in
-// flight at once; then one warp substitutes, lane l holding x of rows l + 32 q (q < 4) in
-// registers and x_j reaching every lane by a shuffle, so no step waits on a CTA barrier.
-// Per row the operations are getrs's, in its order.
-__device__ __forceinline__ double pick4(const double (&v)[4], int q) {
-    return q == 0 ? v[0] : q == 1 ? v[1] : q == 2 ? v[2] : v[3];
-}
-
-__global__ void __launch_bounds__(kTrsvBlk) trsv_diag_kernel(const double* __restrict__ lu, int n, int i0, int bw,
-                                                             bool upper, double* __restrict__ x) {
-    static_assert(kTrsvBlk == 128, "four rows per lane");
-    extern __shared__ double blk[];  // bw x (bw + 1)
-    const int ld = bw + 1;
-    for (int idx = threadIdx.x; idx < bw * bw; idx += blockDim.x) {
-        const int r = idx / bw, c = idx % bw;
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(blk + r * ld + c)),
-                     "l"(lu + (int64_t)(i0 + r) * n + i0 + c)
-                     : "memory");
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-    if (threadIdx.x >= 32) return;
-    const int lane = threadIdx.x;
-    const unsigned full = 0xffffffffu;
-    double v[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] = lane + 32 * q < bw ? x[i0 + lane + 32 * q] : 0.0;
-    if (!upper) {
-#pragma unroll 1
-        for (int j = 0; j < bw; ++j) {
-            const double xj = __shfl_sync(full, pick4(v, j >> 5), j & 31);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int r = lane + 32 * q;
-                if (r > j && r < bw) v[q] -= blk[r * ld + j] * xj;
-            }
-        }
-    } else {
-#pragma unroll 1
-        for (int j = bw - 1; j >= 0; --j) {
-            const int qj = j >> 5;
-            if (lane == (j & 31)) {
-                const double d = blk[j * ld + j];
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (q == qj) v[q] = v[q] / d;
-            }
-            const double xj = __shfl_sync(full, pick4(v, qj), j & 31);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int r = lane + 32 * q;
-                if (r < j) v[q] -= blk[r * ld + j] * xj;
-            }
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-        if (lane + 32 * q < bw) x[i0 + lane + 32 * q] = v[q];
-}
-
-// x[i] -= sum_{j in [j0, j0+bw)} lu[i][j] x[j] for i in [r0, r1): one warp per row.
-__global__ void trsv_update_kernel(const double* __restrict__ lu, int n, int j0, int bw, int r0, int r1,
-                                   double* __restrict__ x) {
-    const int row = r0 + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (row >= r1) return;
-    const double* a = lu + (int64_t)row * n + j0;
-    double acc = 0.0;
-    for (int j = lane; j < bw; j += 32) acc += a[j] * x[j0 + j];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
-    if (lane == 0) x[row] -= acc;
-}
-
-int lu_solve64(const double* lu, int n, const int32_t* piv, double* b, double* work, cudaStream_t s) {
-    if (n <= 0) return fail(FJ_ERR_SHAPE, "lu_solve: n=%d", n);
-    if ((size_t)n * sizeof(int) > 220 * 1024) return fail(FJ_ERR_UNSUPPORTED, "lu_solve: n=%d too large", n);
-    const size_t dsm = (size_t)kTrsvBlk * (kTrsvBlk + 1) * sizeof(double);
-    FJ_TRY(allow_dynamic_smem((const void*)permute_kernel, (size_t)(2 * n * sizeof(int))));
-    FJ_TRY(allow_dynamic_smem((const void*)trsv_diag_kernel, (size_t)dsm));
-    permute_kernel<<<1, 1024, 2 * n * sizeof(int), s>>>(piv, n, b, work); note_launch();
-    const int wpb = 8;
-    for (int i0 = 0; i0 < n; i0 += kTrsvBlk) {  // forward, unit lower
-        const int bw = min(kTrsvBlk, n - i0);
-        trsv_diag_kernel<<<1, kTrsvBlk, (size_t)bw * (bw + 1) * sizeof(double), s>>>(lu, n, i0, bw, false, work); note_launch();
-        const int r0 = i0 + bw;
-        if (r0 < n) {
-            trsv_update_kernel<<<(n - r0 + wpb - 1) / wpb, wpb * 32, 0, s>>>(lu, n, i0, bw, r0, n, work); note_launch();
-        }
-    }
-    for (int i0 = ((n - 1) / kTrsvBlk) * kTrsvBlk; i0 >= 0; i0 -= kTrsvBlk) {  // backward, upper
-        const int bw = min(kTrsvBlk, n - i0);
-        trsv_diag_kernel<<<1, kTrsvBlk, (size_t)bw * (bw + 1) * sizeof(double), s>>>(lu, n, i0, bw, true, work); note_launch();
-        if (i0 > 0) {
-            trsv_update_kernel<<<(i0 + wpb - 1) / wpb, wpb * 32, 0, s>>>(lu, n, i0, bw, 0, i0, work); note_launch();
-        }
-    }
-    FJ_CUDA(cudaMemcpyAsync(b, work, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    FJ_LAUNCH_CHECK("lu_solve64");
-    return FJ_OK;
 }
 
 // ---------------------------------------------------------------------------------
@@ -660,8 +532,8 @@ int lu_inverse32(const float* lu, int n, const int32_t* piv, float* x, cudaStrea
 //
 // lu_factor32_tc: the same partial-pivoting LU, blocked twice.  One launch factors each
 // outer panel of 128 columns (panel_factor; the 16-column panels above where the rows
-// exceed one cluster, their U rows and updates confined to the outer panel).  The columns to its right receive only the row swaps until the outer panel is
-// done; then
+// exceed one cluster, their U rows and updates confined to the outer panel).  The columns to
+// its right receive only the row swaps until the outer panel is done; then
 //   U12 = L11^-1 A12        (lu_trsm32_kernel: forward substitution, CUDA cores, in place)
 //   A22 -= L21 U12          (tensor cores, K = 128)
 //
@@ -869,24 +741,9 @@ int lu_factor32_tc(float* a, int n, int32_t* piv, int* d_info, int* d_err, float
 // Y = P I: row i holds a one in column perm[i].  Y must be zero on entry.
 __global__ void __launch_bounds__(1024) perm_identity_kernel(const int32_t* __restrict__ piv, int n,
                                                              float* __restrict__ y) {
-    extern __shared__ int perm_sm[];  // n permutation entries, then n pivots
-    int* sp = perm_sm + n;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        perm_sm[i] = i;
-        sp[i] = piv[i];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < n; ++i) {
-            const int p = sp[i];
-            if (p != i) {
-                const int t = perm_sm[i];
-                perm_sm[i] = perm_sm[p];
-                perm_sm[p] = t;
-            }
-        }
-    }
-    __syncthreads();
+    extern __shared__ int perm_sm[];
+    __shared__ PermScratch S;
+    build_perm(piv, n, perm_sm, S);
     for (int i = threadIdx.x; i < n; i += blockDim.x) y[(int64_t)i * n + perm_sm[i]] = 1.0f;
 }
 
@@ -900,8 +757,8 @@ int lu_inverse32_tc(const float* lu, int n, const int32_t* piv, float* x, float*
     FJ_TRY(tri_inverse32_blocks(lu, n, 0, nblk, false, tri_l, s));
     FJ_TRY(tri_inverse32_blocks(lu, n, 0, nblk, true, tri_u, s));
     FJ_CUDA(cudaMemsetAsync(x, 0, (size_t)n * n * sizeof(float), s));
-    FJ_TRY(allow_dynamic_smem((const void*)perm_identity_kernel, (size_t)2 * n * sizeof(int)));
-    perm_identity_kernel<<<1, 1024, (size_t)2 * n * sizeof(int), s>>>(piv, n, x);
+    FJ_TRY(allow_dynamic_smem((const void*)perm_identity_kernel, (size_t)n * sizeof(int)));
+    perm_identity_kernel<<<1, 1024, (size_t)n * sizeof(int), s>>>(piv, n, x);
     note_launch();
     FJ_LAUNCH_CHECK("perm_identity_kernel");
     for (int b = 0; b < nblk; ++b) {  // forward: unit lower
