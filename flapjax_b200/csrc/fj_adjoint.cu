@@ -9,16 +9,13 @@
 //     the cutoff kernel :626-648, whose D is |c|^2 and whose pairs within the cutoff
 //     radius of the filament line contribute nothing, derivative included);
 //   * the dense solve (aero/uvlm.py:985) -- A^T mu = lam with the getrf factors of A.
-// K's derivative: with r1 = x - y0, r2 = x - y1, r0 = y1 - y0, c = r1 x r2,
-// u_i = r_i / n_i, n_i = sqrt(|r_i|^2 + eps^2), dot = r0.(u1 - u2), D = |c|^2 + eps|r0|^4,
-// s = dot / (4 pi D), a = lam.c:
-//   d(lam.K)/dr1 = s (r2 x lam) + a [ddot/dr1 - (dot / D) dD/dr1] / (4 pi D)
-//   d(lam.K)/dr2 = s (lam x r1) + a [ddot/dr2 - (dot / D) dD/dr2] / (4 pi D)
-//   ddot/dr1 = (u1 - u2) + (r0 - (r0.u1) u1) / n1,  ddot/dr2 = -(u1 - u2) - (r0 - (r0.u2) u2) / n2
-//   dD/dr1 = 2 (r2 x c) + 4 eps |r0|^2 r0,          dD/dr2 = 2 (c x r1) - 4 eps |r0|^2 r0
-// and x_bar = d/dr1 + d/dr2, y0_bar = -d/dr1, y1_bar = -d/dr2, g_bar = lam.K / g.
+// K's derivative is in fj_bsgrad.cuh; g_bar = lam.K.
+// 2531 targets x 14 118 filaments (cutoff): targets 419 -> 233 us, filaments 467 -> 313 us, of
+// which the FP64 pipe's own 158 and 226 us; 768 x 9 800 (epsilon): 103 -> 63, 106 -> 86 us,
+// against the form with unit vectors and divisions that link_vjp keeps.
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "fj_bsgrad.cuh"
@@ -28,14 +25,17 @@
 namespace fj {
 
 constexpr int kAdjBlock = 128;
+constexpr int kAdjCtas = 4;  // per SM: 8 make two waves; 3 to 6 measured within 5 %, two pairs at a time 10 % faster
 
-// Pass 1: target adjoints.  Walks the stream as the forward sum does.
-template <int KER>
-__global__ void __launch_bounds__(kAdjBlock) vjp_targets_kernel(const double* __restrict__ tgt,
-                                                                const double* __restrict__ lam, int64_t n_t,
-                                                                const Elem64* __restrict__ st, int64_t n_elem,
-                                                                int n_split, double rc2, double* __restrict__ part) {
+// Pass 1: target adjoints.  Walks the stream as the forward sum does.  kAlone: of a call for
+// these only, with the linearisation's arithmetic (link_vjp).
+template <int KER, bool kAlone>
+__global__ void __launch_bounds__(kAdjBlock, kAdjCtas)
+    vjp_targets_kernel(const double* __restrict__ tgt, const double* __restrict__ lam, int64_t n_t,
+                       const Elem64* __restrict__ st, int64_t n_elem, int n_split, double rc2,
+                       double* __restrict__ part) {
     __shared__ Elem64 sh[kAdjBlock];
+    __shared__ double se2[kAdjBlock];
     const int split = blockIdx.y;
     const int64_t per = (n_elem + n_split - 1) / n_split;
     const int64_t e0 = (int64_t)split * per;
@@ -47,36 +47,54 @@ __global__ void __launch_bounds__(kAdjBlock) vjp_targets_kernel(const double* __
     const double lm[3] = {lam[tc * 3], lam[tc * 3 + 1], lam[tc * 3 + 2]};
     double acc[3] = {0.0, 0.0, 0.0};
     if (e0 < e1) {
-        VtxA prev;
-        Elem64 pl = st[e0];
-        vtxa(x, pl.x, pl.y, pl.z, prev);
+        std::conditional_t<kAlone, VtxA, VtxGrad<KER>> prev, v;
+        auto vertex = [&](const Elem64& e, auto& o) {
+            if constexpr (kAlone) vtxa(x, e.x, e.y, e.z, o);
+            else vtx_grad<KER>(x, e.x, e.y, e.z, o);
+        };
+        auto scaled = [&](Elem64 e) {  // (a break's q stays negative)
+            if (kAlone) return e;
+            e.g *= kInv4Pi;
+            if (KER == FJ_KERNEL_CUTOFF) e.q = e.q >= 0.0 ? rc2 * e.q : e.q;
+            return e;
+        };
+        auto e2_of = [](const Elem64& e) { return kEps * kEps * (e.r0x * e.r0x + e.r0y * e.r0y + e.r0z * e.r0z); };
+        Elem64 pl = scaled(st[e0]);
+        double pe2 = e2_of(pl);
+        vertex(pl, prev);
         for (int64_t c0 = e0 + 1; c0 <= vend; c0 += kAdjBlock) {
             const int cnt = (int)min((int64_t)kAdjBlock, vend + 1 - c0);
             __syncthreads();
-            if (threadIdx.x < cnt) sh[threadIdx.x] = st[c0 + threadIdx.x];
+            if (threadIdx.x < cnt) {
+                const Elem64 e = scaled(st[c0 + threadIdx.x]);
+                sh[threadIdx.x] = e;
+                se2[threadIdx.x] = e2_of(e);
+            }
             __syncthreads();
+#pragma unroll 2
             for (int i = 0; i < cnt; ++i) {
                 const Elem64 cur = sh[i];
-                VtxA v;
-                vtxa(x, cur.x, cur.y, cur.z, v);
+                vertex(cur, v);
                 if (pl.q >= 0.0) {
-                    const double r0[3] = {pl.r0x, pl.r0y, pl.r0z};
-                    double g1[3], g2[3], lk;
-                    link_vjp<KER>(prev, v, r0, pl.g, lm, rc2, g1, g2, lk);
-                    acc[0] += g1[0] + g2[0];
-                    acc[1] += g1[1] + g2[1];
-                    acc[2] += g1[2] + g2[2];
+                    if constexpr (kAlone) {
+                        const double r0[3] = {pl.r0x, pl.r0y, pl.r0z};
+                        double g1[3], g2[3], lk;
+                        link_vjp<KER>(prev, v, r0, pl.g, lm, rc2, g1, g2, lk);
+                        for (int k = 0; k < 3; ++k) acc[k] += g1[k] + g2[k];
+                    } else {
+                        const FilGrad f = {{pl.r0x, pl.r0y, pl.r0z}, pl.g, pl.q, pe2};
+                        target_grad<KER>(prev, v, f, rc2, lm, acc);
+                    }
                 }
                 prev = v;
                 pl = cur;
+                pe2 = se2[i];
             }
         }
     }
     if (ti < n_t) {
         double* o = part + ((int64_t)split * n_t + ti) * 3;
-        o[0] = acc[0];
-        o[1] = acc[1];
-        o[2] = acc[2];
+        for (int k = 0; k < 3; ++k) o[k] = acc[k];
     }
 }
 
@@ -84,11 +102,11 @@ __global__ void __launch_bounds__(kAdjBlock) vjp_targets_kernel(const double* __
 // of this CTA's split staged through shared memory.  Output per element and split:
 // [y0_bar(3), y1_bar(3), g_bar].
 template <int KER>
-__global__ void __launch_bounds__(kAdjBlock) vjp_links_kernel(const double* __restrict__ tgt,
-                                                              const double* __restrict__ lam, int64_t n_t,
-                                                              const Elem64* __restrict__ st, int64_t n_elem,
-                                                              int n_split, double rc2, double* __restrict__ part) {
-    __shared__ double sx[kAdjBlock][6];
+__global__ void __launch_bounds__(kAdjBlock, kAdjCtas)
+    vjp_links_kernel(const double* __restrict__ tgt, const double* __restrict__ lam, int64_t n_t,
+                     const Elem64* __restrict__ st, int64_t n_elem, int n_split, double rc2,
+                     double* __restrict__ part) {
+    __shared__ __align__(16) double sx[kAdjBlock][6];
     const int split = blockIdx.y;
     const int64_t per = (n_t + n_split - 1) / n_split;
     const int64_t t0 = (int64_t)split * per;
@@ -103,7 +121,11 @@ __global__ void __launch_bounds__(kAdjBlock) vjp_links_kernel(const double* __re
         memset(&a, 0, sizeof(a));
         memset(&b, 0, sizeof(b));
     }
-    double y0b[3] = {0, 0, 0}, y1b[3] = {0, 0, 0}, gb = 0.0;
+    const double r0sq = a.r0x * a.r0x + a.r0y * a.r0y + a.r0z * a.r0z, e4 = 4.0 * kEps * r0sq;
+    const FilGrad f = {{a.r0x, a.r0y, a.r0z}, kInv4Pi * a.g, KER == FJ_KERNEL_CUTOFF ? rc2 * a.q : a.q,
+                       kEps * kEps * r0sq};
+    LinkGrad l;
+    memset(&l, 0, sizeof(l));
     for (int64_t c0 = t0; c0 < t1; c0 += kAdjBlock) {
         const int cnt = (int)min((int64_t)kAdjBlock, t1 - c0);
         __syncthreads();
@@ -116,30 +138,24 @@ __global__ void __launch_bounds__(kAdjBlock) vjp_links_kernel(const double* __re
         }
         __syncthreads();
         if (live) {
-            const double r0[3] = {a.r0x, a.r0y, a.r0z};
+#pragma unroll 2
             for (int i = 0; i < cnt; ++i) {
                 const double x[3] = {sx[i][0], sx[i][1], sx[i][2]};
                 const double lm[3] = {sx[i][3], sx[i][4], sx[i][5]};
-                VtxA A, B;
-                vtxa(x, a.x, a.y, a.z, A);
-                vtxa(x, b.x, b.y, b.z, B);
-                double g1[3], g2[3], lk;
-                link_vjp<KER>(A, B, r0, a.g, lm, rc2, g1, g2, lk);
-                for (int k = 0; k < 3; ++k) {
-                    y0b[k] -= g1[k];
-                    y1b[k] -= g2[k];
-                }
-                gb += lk;
+                VtxGrad<KER> A, B;
+                vtx_grad<KER>(x, a.x, a.y, a.z, A);
+                vtx_grad<KER>(x, b.x, b.y, b.z, B);
+                link_grad<KER>(A, B, f, rc2, e4, lm, l);
             }
         }
     }
     if (e < n_elem) {
         double* o = part + ((int64_t)split * n_elem + e) * 7;
         for (int k = 0; k < 3; ++k) {
-            o[k] = y0b[k];
-            o[3 + k] = y1b[k];
+            o[k] = -fma(l.e1, f.r0[k], l.d1[k]);
+            o[3 + k] = -fma(l.e2, f.r0[k], l.d2[k]);
         }
-        o[6] = gb;
+        o[6] = kInv4Pi * l.k;
     }
 }
 
@@ -210,9 +226,13 @@ static int64_t vjp_elems(const int* rows, const int* cols, int n_lattices, int i
 }
 
 static int vjp_splits_t(int64_t n_t) { return (int)std::max<int64_t>(1, std::min<int64_t>(64, 1184 / std::max<int64_t>(1, (n_t + kAdjBlock - 1) / kAdjBlock))); }
+// Targets per split of the links' sums, at least: 300 targets, 190 links 33 us with 64, 24 us with
+// 16; more than 2000 targets the same.
+constexpr int kMinTargets = 16;
+
 static int vjp_splits_l(int64_t n_elem, int64_t n_t) {
     const int64_t ctas = (n_elem + kAdjBlock - 1) / kAdjBlock;
-    return (int)std::max<int64_t>(1, std::min<int64_t>({64, 1184 / std::max<int64_t>(1, ctas), std::max<int64_t>(1, n_t / 64)}));
+    return (int)std::max<int64_t>(1, std::min<int64_t>({64, 1184 / std::max<int64_t>(1, ctas), std::max<int64_t>(1, n_t / kMinTargets)}));
 }
 
 }  // namespace fj
@@ -295,12 +315,13 @@ int fj_vind_vjp(const double* d_targets, int64_t n_targets, const double* const*
     FJ_TRY(pack_stream64(pa, st, s));
     if (d_targets_bar) {
         dim3 g((unsigned)((n_targets + kAdjBlock - 1) / kAdjBlock), (unsigned)st_split);
-        if (kernel == FJ_KERNEL_EPSILON)
-            vjp_targets_kernel<FJ_KERNEL_EPSILON><<<g, kAdjBlock, 0, s>>>(d_targets, d_lam, n_targets, st, ne,
-                                                                          st_split, rc2, part_t);
-        else
-            vjp_targets_kernel<FJ_KERNEL_CUTOFF><<<g, kAdjBlock, 0, s>>>(d_targets, d_lam, n_targets, st, ne,
-                                                                         st_split, rc2, part_t);
+        const bool alone = d_zetas_bar == nullptr && d_gammas_bar == nullptr;
+        auto* fn = kernel == FJ_KERNEL_EPSILON
+                       ? (alone ? vjp_targets_kernel<FJ_KERNEL_EPSILON, true>
+                                : vjp_targets_kernel<FJ_KERNEL_EPSILON, false>)
+                       : (alone ? vjp_targets_kernel<FJ_KERNEL_CUTOFF, true>
+                                : vjp_targets_kernel<FJ_KERNEL_CUTOFF, false>);
+        fn<<<g, kAdjBlock, 0, s>>>(d_targets, d_lam, n_targets, st, ne, st_split, rc2, part_t);
         note_launch();
         sum_splits_kernel<<<(unsigned)((n_targets * 3 + 255) / 256), 256, 0, s>>>(part_t, st_split, n_targets * 3,
                                                                                  d_targets_bar, 1); note_launch();
@@ -314,7 +335,7 @@ int fj_vind_vjp(const double* d_targets, int64_t n_targets, const double* const*
             vjp_links_kernel<FJ_KERNEL_CUTOFF><<<g, kAdjBlock, 0, s>>>(d_targets, d_lam, n_targets, st, ne, l_split,
                                                                        rc2, part_l);
         note_launch();
-        sum_splits_kernel<<<(unsigned)((ne * 7 + 255) / 256), 256, 0, s>>>(part_l, l_split, ne * 7, el, 0); note_launch();
+        FJ_TRY(reduce_sums(part_l, l_split, ne * 7, el, 0, 1.0, s));
         for (int li = 0; li < n; ++li) {
             const int64_t nv = (int64_t)(ua.lat[li].rows + 1) * (ua.lat[li].cols + 1);
             if (ua.zeta_bar[li]) {

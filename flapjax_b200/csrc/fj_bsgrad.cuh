@@ -1,25 +1,156 @@
 // fj_bsgrad.cuh -- derivatives of one Biot-Savart filament (FP64), shared by the
 // adjoint sums (fj_adjoint.cu) and the dense influence Jacobians (fj_jac.cu).
 //
-// With r1 = x - y0, r2 = x - y1, r0 = y1 - y0 = r1 - r2, c = r1 x r2,
-// u_i = r_i / n_i, n_i = sqrt(|r_i|^2 + eps^2), dot = r0.(u1 - u2), D = |c|^2 + eps|r0|^4
-// (epsilon kernel, aero/utils.py:606-623) or |c|^2 (cutoff kernel, :626-648, whose pairs
-// within the cutoff radius of the filament line contribute nothing, derivative included),
-// s = dot / (4 pi D), a = lam.c:
-//   d(lam.K)/dr1 = s (r2 x lam) + a [ddot/dr1 - (dot / D) dD/dr1] / (4 pi D)
-//   d(lam.K)/dr2 = s (lam x r1) + a [ddot/dr2 - (dot / D) dD/dr2] / (4 pi D)
-//   ddot/dr1 = (u1 - u2) + (r0 - (r0.u1) u1) / n1,  ddot/dr2 = -(u1 - u2) - (r0 - (r0.u2) u2) / n2
-//   dD/dr1 = 2 (r2 x c) + 4 eps |r0|^2 r0,          dD/dr2 = 2 (c x r1) - 4 eps |r0|^2 r0
-// and x_bar = d/dr1 + d/dr2, y0_bar = -d/dr1, y1_bar = -d/dr2.
+// With r1 = x - y0, r2 = x - y1, r0 = y1 - y0 = r1 - r2, c = r1 x r2, n_i = sqrt(|r_i|^2 + eps^2),
+// dot = r0.(r1 / n1 - r2 / n2), D = |c|^2 + eps|r0|^4 (epsilon kernel, aero/utils.py:606-623) or
+// |c|^2 (cutoff kernel, :626-648, whose pairs within the cutoff radius of the filament line
+// contribute nothing, derivative included), s = dot / D, b = (lam.c) / D and w = lam - 2 b c, the
+// derivatives of 4 pi lam.K = s (lam.c) are
+//   d/dr1 = s (r2 x w) + b [r1/n1 - r2/n2 + r0/n1 - (r0.r1/n1^3) r1] - 4 eps b s |r0|^2 r0
+//   d/dr2 = s (w x r1) - b [r1/n1 - r2/n2 + r0/n2 - (r0.r2/n2^3) r2] + 4 eps b s |r0|^2 r0
+// (w carries both the cross products' and |c|^2's), and for the target
+//   d/dr1 + d/dr2 = s (w x r0) + b [(1/n1 - 1/n2) r0 - (r0.r1/n1^3) r1 + (r0.r2/n2^3) r2].
+// x_bar = d/dr1 + d/dr2, y0_bar = -d/dr1, y1_bar = -d/dr2.
+//
+// As the sums themselves these are bound by the FP64 pipe and written for few operations: per
+// pair 80 for the target and 114 for the filament's two ends and strength (which has both
+// vertices to itself), one reciprocal square root a vertex and one reciprocal a filament
+// (fj_bs.cuh), the cutoff's radius test on the integer pipe.
+//
+// dot: a target on the filament's line but beyond its ends has r1 / n1 = r2 / n2, and its
+// derivative, unlike its velocity, keeps dot's rounding whole, over a D of eps|r0|^4 alone.  With
+// P = r1.r2 + eps^2, dot = (1/n1 + 1/n2) (n1 n2 - P), and where P > 0 (no end between)
+// n1 n2 - P = (|c|^2 + eps^2 |r0|^2) / (n1 n2 + P), in which nothing cancels.
 #pragma once
 
-#include "fj_common.cuh"
+#include "fj_bs.cuh"
 
 namespace fj {
 
-// Per vertex one reciprocal square root and per link one division (1 / (4 pi D)); the
-// other quotients are products with these reciprocals (the FP64 divide and square root
-// are multi-instruction sequences on the FP64 pipe).
+template <int KER>
+struct VtxGrad {
+    double d[3], inv, inv2, n;  // x - y; 1 / n, 1 / n^2, n
+};
+
+template <int KER>
+__device__ __forceinline__ void vtx_grad(const double x[3], double yx, double yy, double yz, VtxGrad<KER>& o) {
+    o.d[0] = x[0] - yx;
+    o.d[1] = x[1] - yy;
+    o.d[2] = x[2] - yz;
+    const double n2 = fma(o.d[2], o.d[2], fma(o.d[1], o.d[1], fma(o.d[0], o.d[0], kEps * kEps)));
+    o.inv = rsqrt_normal(n2);
+    o.inv2 = o.inv * o.inv;
+    o.n = n2 * o.inv;
+}
+
+// (Written out: the two passes' products are to round alike, see LinkGrad.)
+__device__ __forceinline__ void cross_grad(const double a[3], const double b[3], double (&o)[3]) {
+    o[0] = fma(a[1], b[2], -(a[2] * b[1]));
+    o[1] = fma(a[2], b[0], -(a[0] * b[2]));
+    o[2] = fma(a[0], b[1], -(a[1] * b[0]));
+}
+
+__device__ __forceinline__ double dot_grad(const double a[3], const double b[3], double c) {
+    return fma(a[2], b[2], fma(a[1], b[1], fma(a[0], b[0], c)));
+}
+
+// A filament: vector, strength / (4 pi), the kernel's q (see link64), eps^2 |r0|^2.
+struct FilGrad {
+    double r0[3], g, q, e2;
+};
+
+// What both derivatives take from a pair: g s, g b, w; s1, s2 = r0.r_i / n_i^2; k = s (lam.c).
+struct PairGrad {
+    double gs, gb, s1, s2, w[3], s, k;
+};
+
+template <int KER>
+__device__ __forceinline__ void pair_grad(const VtxGrad<KER>& A, const VtxGrad<KER>& B, const FilGrad& f, double rc2,
+                                          const double lam[3], PairGrad& o) {
+    static_assert(KER != FJ_KERNEL_PLAIN, "the plain kernel has no adjoint");
+    double c[3];
+    cross_grad(A.d, B.d, c);
+    const double c2 = dot_grad(c, c, 0.0);
+    const double P = dot_grad(A.d, B.d, kEps * kEps), Z = fma(A.n, B.n, fabs(P));
+    const bool ahead = __double2hiint(P) > 0;
+    const double D = KER == FJ_KERNEL_EPSILON ? c2 + f.q : c2;
+    const double num = ahead ? c2 + f.e2 : Z, den = ahead ? Z : 1.0;
+    const double inv = rcp_normal(den * D);
+    double a = dot_grad(lam, c, 0.0), b = a * (den * inv);
+    o.s = (A.inv + B.inv) * num * inv;
+    o.s1 = A.inv2 * dot_grad(f.r0, A.d, 0.0);
+    o.s2 = B.inv2 * dot_grad(f.r0, B.d, 0.0);
+    if (KER == FJ_KERNEL_CUTOFF) {
+        bool close = false, keep = outside_core(c2, f.q, close);
+        if (close) {
+            keep = outside_core(A.d, f.r0[0], f.r0[1], f.r0[2], rc2);
+            if (!keep) a = c[0] = c[1] = c[2] = 0.0;  // (they may be NaN)
+        }
+        o.s = keep ? o.s : 0.0;
+        b = keep ? b : 0.0;
+    }
+    o.k = o.s * a;
+    o.gs = f.g * o.s;
+    o.gb = f.g * b;
+    const double b2 = -2.0 * b;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) o.w[k] = fma(b2, c[k], lam[k]);
+}
+
+// acc += g d(lam.K)/dx, the pair's terms added up before (acc may be of the size of 1 / (eps
+// |r0|^3), see LinkGrad, and a rounding of that size a pair is enough).
+template <int KER>
+__device__ __forceinline__ void target_grad(const VtxGrad<KER>& A, const VtxGrad<KER>& B, const FilGrad& f, double rc2,
+                                            const double lam[3], double (&acc)[3]) {
+    PairGrad p;
+    pair_grad<KER>(A, B, f, rc2, lam, p);
+    const double f1 = p.gb * A.inv, f2 = p.gb * B.inv, h0 = f1 - f2, h1 = f1 * p.s1, h2 = f2 * p.s2;
+    double t[3];
+    cross_grad(p.w, f.r0, t);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        acc[i] += fma(p.gs, t[i], fma(h0, f.r0[i], fma(-h1, A.d[i], h2 * B.d[i])));
+}
+
+// The sums over targets of one filament's derivatives, but for its vector in the terms along
+// it: g d(lam.K)/dr1 = d1 + e1 r0, likewise d2, e2; k: 4 pi lam.K.  g goes into s and b first, as
+// for the target: a filament of a surface and the target at its middle, which moves with it,
+// have derivatives of 1 / (eps |r0|^3) that cancel, and so do their roundings where both are
+// made of the same products.
+struct LinkGrad {
+    double d1[3], d2[3], e1, e2, k;
+};
+
+// e4 = 4 eps |r0|^2 (epsilon kernel).
+template <int KER, bool kEnd1 = true, bool kEnd2 = true>
+__device__ __forceinline__ void link_grad(const VtxGrad<KER>& A, const VtxGrad<KER>& B, const FilGrad& f, double rc2,
+                                          double e4, const double lam[3], LinkGrad& o) {
+    PairGrad p;
+    pair_grad<KER>(A, B, f, rc2, lam, p);
+    const double f1 = p.gb * A.inv, f2 = p.gb * B.inv;
+    const double se = KER == FJ_KERNEL_EPSILON ? p.s * e4 : 0.0;
+    double t[3];
+    if (kEnd1) {
+        const double h = fma(-f1, p.s1, f1);
+        cross_grad(B.d, p.w, t);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) o.d1[i] += fma(p.gs, t[i], fma(h, A.d[i], -f2 * B.d[i]));
+        o.e1 = KER == FJ_KERNEL_EPSILON ? fma(p.gb, A.inv - se, o.e1) : o.e1 + f1;
+    }
+    if (kEnd2) {
+        const double h = fma(f2, p.s2, f2);
+        cross_grad(p.w, A.d, t);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) o.d2[i] += fma(p.gs, t[i], fma(-f1, A.d[i], h * B.d[i]));
+        o.e2 = KER == FJ_KERNEL_EPSILON ? fma(p.gb, se - B.inv, o.e2) : o.e2 - f2;
+    }
+    o.k += p.k;
+}
+
+// The same derivatives for the linearisation, by the unit vectors and per end in full.  It adds
+// the targets' to the vertices' (fj_vertex_jacobian) where a target moves with a filament, and
+// the entries of 1 / (eps |r0|^3) that cancel there leave 1e-9 of themselves: one arithmetic for
+// both, whose cost (180 operations a pair) its host work hides.
 struct VtxA {
     double d[3];  // x - y
     double u[3];  // d / n

@@ -760,10 +760,13 @@ int reduce_jobs(const VindJob* d_jobs, int n_jobs, int64_t max_targets, cudaStre
 
 int reduce_partials(const double* part, int n_part, int64_t n_targets, double* out, int accumulate,
                     double scale, cudaStream_t s) {
-    const int64_t n3 = n_targets * 3;
-    if (n3 == 0) return FJ_OK;
-    reduce_partials_kernel<<<(unsigned)((n3 + kRedOut - 1) / kRedOut), kRedOut * kRedLanes, 0, s>>>(
-        part, n_part, n3, out, accumulate, scale); note_launch();
+    return reduce_sums(part, n_part, n_targets * 3, out, accumulate, scale, s);
+}
+
+int reduce_sums(const double* part, int n_part, int64_t n, double* out, int accumulate, double scale, cudaStream_t s) {
+    if (n == 0) return FJ_OK;
+    reduce_partials_kernel<<<(unsigned)((n + kRedOut - 1) / kRedOut), kRedOut * kRedLanes, 0, s>>>(
+        part, n_part, n, out, accumulate, scale); note_launch();
     FJ_LAUNCH_CHECK("reduce_partials_kernel");
     return FJ_OK;
 }

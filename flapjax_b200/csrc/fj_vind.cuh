@@ -110,6 +110,8 @@ inline int64_t lattice_links(int rows, int cols) {
 int vind_launch(const VindJob& job, int precision, int kernel, double r_cut, cudaStream_t s, int tile = 0);
 int reduce_partials(const double* part, int n_part, int64_t n_targets, double* out,
                     int accumulate, double scale, cudaStream_t s);
+// The same of n outputs of any kind.
+int reduce_sums(const double* part, int n_part, int64_t n, double* out, int accumulate, double scale, cudaStream_t s);
 int choose_split(int64_t n_targets, int64_t n_elem, int precision);
 // FP32 targets per thread for a shape: 4 where the autotuner found the wide tile faster,
 // else 2 (FP64: 2).
