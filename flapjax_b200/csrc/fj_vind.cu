@@ -429,10 +429,16 @@ __global__ void __launch_bounds__(kBlock, kMinCtas64) vind64_kernel(VindJob job,
 // FP32 sum.
 // ------------------------------------------------------------------------------------
 // Packed form: two targets ride in one float2 and every FP32 add/mul/fma of the pair is
-// one f32x2 instruction (sm_100: __fadd2_rn / __fmul2_rn / __ffma2_rn), halving the
-// issue slots per pair of the scalar form.  The staged element is stored duplicated in
-// shared memory ({v, v} pairs, 7 float4), so the broadcast loads give packed operands
-// directly.  Subtractions are fma(b, -1, a), which is exact.  T = 2 P targets per thread.
+// one f32x2 instruction (sm_100: __fadd2_rn / __fmul2_rn / __ffma2_rn).  Such an instruction
+// takes two issue slots, and the slots bound the sum: 38 (cutoff; epsilon 40) packed ones and
+// 33 others made 109 of the 111 slots a packed pair took.  So the others count as much, and
+// what a product by a selected factor would cost in selects a predicated scalar product saves:
+// 25 800 targets x 55 600 filaments, cutoff 2206 -> 2092 us (6.9e11 pairs/s), epsilon 2203 ->
+// 2163 us.  The scalar form, bit for bit the same, has fewer instructions (its negations and
+// absolute values are operand modifiers) and loses one issue in seven: 2296 us.  The staged
+// element is stored duplicated in shared memory ({v, v} pairs, 7 float4), so the broadcast
+// loads give packed operands directly.  Subtractions are fma(b, -1, a), which is exact.
+// T = 2 P targets per thread.
 //
 // Cancellation-free strength.  The reference's factor r0 . (r1/|r1| - r2/|r2|) subtracts
 // two nearly equal unit vectors whenever the target is far from the filament compared with
@@ -510,11 +516,29 @@ __device__ __forceinline__ void vtx32x2(const float2 xh[3], const float2 xl[3], 
     o.s = make_float2(n2.x > e2 ? s.x : __int_as_float(0x7f800000), n2.y > e2 ? s.y : __int_as_float(0x7f800000));
 }
 
+// Q where D > 0, else v into o, and f *= Q on the other side: products by a selected one would
+// cost a select and a slot more (fma.rn.f32x2 takes two).
+__device__ __forceinline__ void ahead_cut(float D, float Q, float v, float& f, float& o) {
+    asm("{\n.reg .pred p;\nsetp.gt.f32 p, %2, 0f00000000;\n@!p mul.rn.f32 %0, %0, %3;\nselp.f32 %1, %3, %4, p;\n}"
+        : "+f"(f), "=f"(o)
+        : "f"(D), "f"(Q), "f"(v));
+}
+
+__device__ __forceinline__ void ahead_eps(float D, float Q, float v, float& f, float& o) {
+    asm("{\n.reg .pred p;\nsetp.gt.f32 p, %2, 0f00000000;\n@p mul.rn.f32 %0, %0, %3;\nselp.f32 %1, %4, %3, p;\n}"
+        : "+f"(f), "=f"(o)
+        : "f"(D), "f"(Q), "f"(v));
+}
+
+// o = x y where c > m.
+__device__ __forceinline__ void mul_if_above(float c, float m, float x, float y, float& o) {
+    asm("{\n.reg .pred p;\nsetp.gt.f32 p, %1, %2;\n@p mul.rn.f32 %0, %3, %4;\n}" : "+f"(o) : "f"(c), "f"(m), "f"(x), "f"(y));
+}
+
 // The link from vertex a (element e) to vertex b (element e+1) with element e's link part l.
 template <int KER>
 __device__ __forceinline__ void link32x2(const Vtx32x2& a, const Vtx32x2& b, const float4* __restrict__ l,
                                          float2 acc[3]) {
-    const float2 neg1 = dup2(-1.0f);
     const float4 l0 = l[0], l1 = l[1], l2 = l[2], l3 = l[3];
     const float2 g = make_float2(l0.x, l0.y), q = make_float2(l0.z, l0.w);
     const float2 r0x = make_float2(l1.x, l1.y), r0y = make_float2(l1.z, l1.w), r0z = make_float2(l2.x, l2.y);
@@ -525,25 +549,25 @@ __device__ __forceinline__ void link32x2(const Vtx32x2& a, const Vtx32x2& b, con
     const float2 c2 = __ffma2_rn(cz, cz, __ffma2_rn(cy, cy, __fmul2_rn(cx, cx)));
     const float2 D = __ffma2_rn(a.d[2], b.d[2], __ffma2_rn(a.d[1], b.d[1], __fmul2_rn(a.d[0], b.d[0])));
     const float2 P = __fmul2_rn(a.n, b.n);
-    const float2 PpD = __fadd2_rn(P, D);
-    const float2 PmD = __ffma2_rn(D, neg1, P);
     const float2 t = __fmul2_rn(a.s, b.s);
-    const float2 gS = __fmul2_rn(g, __fadd2_rn(a.n, b.n));
-    float2 coef;
+    float2 gS = __fmul2_rn(g, __fadd2_rn(a.n, b.n)), coef = make_float2(0.0f, 0.0f), den;
+    // P + D where D > 0, P - D elsewhere
+    const float2 Q = make_float2(__fadd_rn(P.x, fabsf(D.x)), __fadd_rn(P.y, fabsf(D.y)));
     if (KER == FJ_KERNEL_EPSILON) {
-        const float2 N = make_float2(D.x > 0.0f ? c2.x : PmD.x, D.y > 0.0f ? c2.y : PmD.y);
-        const float2 M = make_float2(D.x > 0.0f ? PpD.x : 1.0f, D.y > 0.0f ? PpD.y : 1.0f);
-        const float2 den = __fmul2_rn(__fmul2_rn(P, M), __fadd2_rn(c2, q));
-        coef = __fmul2_rn(__fmul2_rn(gS, N), make_float2(rcp_ftz(den.x), rcp_ftz(den.y)));
-        coef.x = c2.x > t.x ? coef.x : 0.0f;
-        coef.y = c2.y > t.y ? coef.y : 0.0f;
+        float2 N, PM = P;
+        ahead_eps(D.x, Q.x, c2.x, PM.x, N.x);
+        ahead_eps(D.y, Q.y, c2.y, PM.y, N.y);
+        den = __fmul2_rn(PM, __fadd2_rn(c2, q));
+        gS = __fmul2_rn(gS, N);
+        mul_if_above(c2.x, t.x, gS.x, rcp_ftz(den.x), coef.x);
+        mul_if_above(c2.y, t.y, gS.y, rcp_ftz(den.y), coef.y);
     } else {
-        const float2 X = make_float2(D.x > 0.0f ? 1.0f : PmD.x, D.y > 0.0f ? 1.0f : PmD.y);
-        const float2 Y = make_float2(D.x > 0.0f ? PpD.x : c2.x, D.y > 0.0f ? PpD.y : c2.y);
-        const float2 den = __fmul2_rn(P, Y);
-        coef = __fmul2_rn(__fmul2_rn(gS, X), make_float2(rcp_ftz(den.x), rcp_ftz(den.y)));
-        coef.x = c2.x > fmaxf(q.x, t.x) ? coef.x : 0.0f;
-        coef.y = c2.y > fmaxf(q.y, t.y) ? coef.y : 0.0f;
+        float2 Y;
+        ahead_cut(D.x, Q.x, c2.x, gS.x, Y.x);
+        ahead_cut(D.y, Q.y, c2.y, gS.y, Y.y);
+        den = __fmul2_rn(P, Y);
+        mul_if_above(c2.x, fmaxf(q.x, t.x), gS.x, rcp_ftz(den.x), coef.x);
+        mul_if_above(c2.y, fmaxf(q.y, t.y), gS.y, rcp_ftz(den.y), coef.y);
     }
     acc[0] = __ffma2_rn(cx, coef, acc[0]);
     acc[1] = __ffma2_rn(cy, coef, acc[1]);
