@@ -158,45 +158,59 @@ struct StepCase {
     double polar_scale;     // polar_circulation_scale
 };
 
-// Also clears the lattice-changed flag that k_changed sets later in the step (nothing in
-// between reads it).
-__global__ void k_time(const StepCase* __restrict__ T) {
-    const StepCase& C = T[blockIdx.y];
-    if (threadIdx.x == 0 && C.advance_time && C.i > 0) C.t[C.i] = C.t[C.i - 1] + C.dt;  // uvlm.py:1158-1161
-    if (threadIdx.x == 0 && C.changed != nullptr) *C.changed = 0;
+// The small kernels of a step take 2 to 4 us each, all of it latency (of the table, of the
+// arrays it names, and of the launch), so what may run side by side shares a launch: a kernel
+// of several parts gives each a range of blocks.  A step of an 8 x 32 wing, 34 launches: 148 us
+// (mixed) and 336 us (FP64); these parts together, 27 launches: 129 and 316 us.  Letting each
+// launch begin while the one before ends (programmatic dependent launch) gave 145 us.
+struct Parts {
+    unsigned end[5];  // block after each part's last
+};
+
+__device__ __forceinline__ int64_t part_index(const Parts& parts, int q) {
+    return (int64_t)(blockIdx.x - (q > 0 ? parts.end[q - 1] : 0)) * blockDim.x + threadIdx.x;
 }
 
-// hg_to_zeta_b / hg_dot_to_zeta_b_dot (aero/uvlm.py:537-621), one thread per vertex.
-__global__ void k_geom_vertices(const StepCase* __restrict__ T) {
+// hg_to_zeta_b / hg_dot_to_zeta_b_dot (aero/uvlm.py:537-621), one thread per vertex; the first
+// one also advances the time and clears the lattice-changed flag that k_lattice sets later in the
+// step.  All loads are issued before the first store, which might alias them.
+__global__ void k_vertices(const StepCase* __restrict__ T) {
     const StepCase& C = T[blockIdx.y];
     const Layout& L = C.L;
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= L.vo[L.n_surf]) return;
     const int s = find_surf(L.vo, L.n_surf, v);
-    const int j = (int)((v - L.vo[s]) % (L.n[s] + 1));
+    const int j = (int)(v - L.vo[s]) % (L.n[s] + 1);
     // the host validates the mapping; the clamp only keeps a bad entry in bounds
-    const int node = min(max(C.dof[L.dofo[s] + j], 0), L.n_nodes - 1);
+    const int64_t node = min(max(C.dof[L.dofo[s] + j], 0), L.n_nodes - 1);
     const double x0[3] = {C.zeta0[v * 3], C.zeta0[v * 3 + 1], C.zeta0[v * 3 + 2]};
-    double o[3];
-    se3_apply(C.hg_n + (int64_t)node * 16, x0, o);
-    for (int d = 0; d < 3; ++d) C.zb_n[v * 3 + d] = o[d];
-    if (C.hgd_n != nullptr) {
-        se3_apply(C.hgd_n + (int64_t)node * 16, x0, o);
-    } else {
-        o[0] = o[1] = o[2] = 0.0;
+    const double* src[3] = {C.hg_n, C.hgd_n, C.hg_nm1};
+    double* dst[3] = {C.zb_n, C.zbd_n, C.zb_nm1};
+    double hg[3][12];
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+#pragma unroll
+        for (int e = 0; e < 12; ++e) hg[q][e] = src[q] != nullptr ? src[q][node * 16 + e] : 0.0;
+    double* t = C.t;
+    int* changed = C.changed;
+    const int i = C.i, advance = C.advance_time;
+    const double dt = C.dt;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        double o[3];
+        se3_apply(hg[q], x0, o);
+        if (q == 2 && src[2] == nullptr) break;
+        for (int d = 0; d < 3; ++d) dst[q][v * 3 + d] = src[q] != nullptr ? o[d] : 0.0;
     }
-    for (int d = 0; d < 3; ++d) C.zbd_n[v * 3 + d] = o[d];
-    if (C.hg_nm1 != nullptr) {
-        se3_apply(C.hg_nm1 + (int64_t)node * 16, x0, o);
-        for (int d = 0; d < 3; ++d) C.zb_nm1[v * 3 + d] = o[d];
+    if (v == 0) {
+        if (advance && i > 0) t[i] = t[i - 1] + dt;  // uvlm.py:1158-1161
+        if (changed != nullptr) *changed = 0;
     }
 }
 
 // compute_surf_c / compute_surf_nc (aero/utils.py:87-105) and c_dot (uvlm.py:891-893).
-__global__ void k_geom_panels(const StepCase* __restrict__ T) {
-    const StepCase& C = T[blockIdx.y];
+__device__ __forceinline__ void geom_panel(const StepCase& C, const int64_t p) {
     const Layout& L = C.L;
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= L.po[L.n_surf]) return;
     const int s = find_surf(L.po, L.n_surf, p);
     const int64_t lp = p - L.po[s];
@@ -275,11 +289,9 @@ __global__ void init_wake_kernel(Layout L, const double* __restrict__ zeta_b, fj
 }
 
 // Rows 0..m_star-1 of every surface's wake at n-1, packed as the free-wake target list.
-__global__ void k_gather_wake_targets(const StepCase* __restrict__ T) {
-    const StepCase& C = T[blockIdx.y];
+__device__ __forceinline__ void gather_wake_target(const StepCase& C, const int64_t t) {
     const Layout& L = C.L;
     if (!C.free_wake) return;
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= L.wto[L.n_surf]) return;
     const int s = find_surf(L.wto, L.n_surf, t);
     const int64_t src = L.wvo[s] + (t - L.wto[s]);
@@ -288,10 +300,8 @@ __global__ void k_gather_wake_targets(const StepCase* __restrict__ T) {
 
 // propagate_surf_wake, uniform branch (aero/utils.py:427-450): shed the TE row and
 // circulation of step n-1, drop the last row, convect the rest by dt * (U + v_ind).
-__global__ void k_wake_shed(const StepCase* __restrict__ T) {
-    const StepCase& C = T[blockIdx.y];
+__device__ __forceinline__ void wake_shed(const StepCase& C, const int64_t v) {
     const Layout& L = C.L;
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t nv = L.wvo[L.n_surf];
     const double t = C.t[C.i];
     if (v < nv) {
@@ -468,10 +478,8 @@ __global__ void static_gamma_w_kernel(Layout L, const double* __restrict__ gamma
 }
 
 // Mixed path: flag a lattice that differs (bitwise) from the one of the cached AIC.
-__global__ void k_changed(const StepCase* __restrict__ T) {
-    const StepCase& C = T[blockIdx.y];
+__device__ __forceinline__ void compare_lattice(const StepCase& C, const int64_t i) {
     if (C.changed == nullptr) return;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < C.L.vo[C.L.n_surf] * 3 && C.zb_n[i] != C.zeta_ref[i]) *C.changed = 1;
 }
 
@@ -517,10 +525,8 @@ __device__ __forceinline__ void filament_ends(const Layout& L, int s, int64_t lf
     }
 }
 
-__global__ void k_force_targets(const StepCase* __restrict__ T) {
-    const StepCase& C = T[blockIdx.y];
+__device__ __forceinline__ void force_target(const StepCase& C, const int64_t fi) {
     const Layout& L = C.L;
-    const int64_t fi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (fi >= L.fo[L.n_surf]) return;
     const int s = find_surf(L.fo, L.n_surf, fi);
     int k0, l0, k1, l1;
@@ -532,10 +538,21 @@ __global__ void k_force_targets(const StepCase* __restrict__ T) {
     for (int d = 0; d < 3; ++d) C.targets[fi * 3 + d] = 0.5 * (a[d] + b[d]);
 }
 
-__global__ void k_force_filament(const StepCase* __restrict__ T) {
+// What follows from the lattice alone: the panels, the comparison with the cached AIC's lattice,
+// the free wake's targets, the shed wake and the force targets.  Where a wake convects freely the
+// last two come later (k_lattice again, the first parts empty): they wait for the wake's
+// velocities, whose targets lie where the force targets come to.
+__global__ void k_lattice(const StepCase* __restrict__ T, Parts parts) {
     const StepCase& C = T[blockIdx.y];
+    if (blockIdx.x < parts.end[0]) geom_panel(C, part_index(parts, 0));
+    else if (blockIdx.x < parts.end[1]) compare_lattice(C, part_index(parts, 1));
+    else if (blockIdx.x < parts.end[2]) gather_wake_target(C, part_index(parts, 2));
+    else if (blockIdx.x < parts.end[3]) wake_shed(C, part_index(parts, 3));
+    else force_target(C, part_index(parts, 4));
+}
+
+__device__ __forceinline__ void force_filament(const StepCase& C, const int64_t fi) {
     const Layout& L = C.L;
-    const int64_t fi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (fi >= L.fo[L.n_surf]) return;
     const double t = C.t[C.i];
     const int s = find_surf(L.fo, L.n_surf, fi);
@@ -573,13 +590,18 @@ __global__ void k_force_filament(const StepCase* __restrict__ T) {
 }
 
 // compute_gamma_dot (uvlm.py:691-715)
-__global__ void k_gamma_dot(const StepCase* __restrict__ T) {
-    const StepCase& C = T[blockIdx.y];
+__device__ __forceinline__ void gamma_dot(const StepCase& C, const int64_t p) {
     if (C.gbd_nm1 == nullptr) return;
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= C.nb) return;
     const double cur = (C.gb_n[p] - C.gb_nm1[p]) / C.dt;
     C.gbd_n[p] = cur * C.relax + C.gbd_nm1[p] * (1.0 - C.relax);
+}
+
+// The filament forces and gamma_dot.
+__global__ void k_filaments(const StepCase* __restrict__ T, Parts parts) {
+    const StepCase& C = T[blockIdx.y];
+    if (blockIdx.x < parts.end[0]) force_filament(C, part_index(parts, 0));
+    else gamma_dot(C, part_index(parts, 1));
 }
 
 // split_to_vertex of the filament forces (aero/utils.py:220-222) and of
@@ -627,10 +649,8 @@ __global__ void k_vertex_forces(const StepCase* __restrict__ T, int parts) {
 }
 
 // strip_alpha (aero/utils.py:226-273), one thread per strip.
-__global__ void k_strip_alpha(const StepCase* __restrict__ T) {
-    const StepCase& C = T[blockIdx.y];
+__device__ __forceinline__ void strip_alpha(const StepCase& C, const int64_t j) {
     const Layout& L = C.L;
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= L.so[L.n_surf]) return;
     const double t = C.t[C.i];
     const int s = find_surf(L.so, L.n_surf, j);
@@ -798,8 +818,7 @@ __global__ void k_polar_gamma(const StepCase* __restrict__ T) {
 }
 
 // Sum over vertices of f_steady + f_unsteady (one CTA per case, fixed order).
-__global__ void k_force_total(const StepCase* __restrict__ T) {
-    const StepCase& C = T[blockIdx.y];
+__device__ __forceinline__ void force_total(const StepCase& C) {
     const int64_t nv = C.L.vo[C.L.n_surf];
     __shared__ double sh[3][256];
     double a[3] = {0.0, 0.0, 0.0};
@@ -820,7 +839,32 @@ __global__ void k_force_total(const StepCase* __restrict__ T) {
     }
 }
 
+// The strips' angles and the total force.
+__global__ void k_strips(const StepCase* __restrict__ T, Parts parts) {
+    const StepCase& C = T[blockIdx.y];
+    if (blockIdx.x < parts.end[0]) strip_alpha(C, part_index(parts, 0));
+    else force_total(C);
+}
+
+static Parts parts_of(std::initializer_list<unsigned> blocks) {
+    Parts p = {};
+    unsigned end = 0;
+    int q = 0;
+    for (unsigned n : blocks) p.end[q++] = end += n;
+    for (; q < 5; ++q) p.end[q] = end;
+    return p;
+}
+
 static inline unsigned nblk(int64_t n, int b = 256) { return (unsigned)((n + b - 1) / b); }
+
+// A kernel of several parts over K cases, each part's blocks given.
+static void launch_parts(void (*fn)(const StepCase*, Parts), std::initializer_list<unsigned> blocks, int K,
+                         const StepCase* dC, cudaStream_t s) {
+    const Parts p = parts_of(blocks);
+    if (p.end[4] == 0) return;
+    fn<<<dim3(p.end[4], (unsigned)K), 256, 0, s>>>(dC, p);
+    note_launch();
+}
 
 // ------------------------------------------------------------------------------------
 // Case plan: layout, workspace carve-up, validation
@@ -1232,8 +1276,8 @@ static int run_static(const Plan& p, const fj_case_buffers* B, const double* hg,
     const TableLayout tl = table_layout(1);
     StepCase* dC = (StepCase*)(p.tab + tl.step);
     FJ_TRY(upload(dC, &C, sizeof(C), s));
-    k_geom_vertices<<<nblk(L.vo[L.n_surf]), 256, 0, s>>>(dC); note_launch();
-    k_geom_panels<<<nblk(L.po[L.n_surf]), 256, 0, s>>>(dC); note_launch();
+    k_vertices<<<nblk(L.vo[L.n_surf]), 256, 0, s>>>(dC); note_launch();
+    launch_parts(k_lattice, {nblk(L.po[L.n_surf]), 0, 0, 0, nblk(L.fo[L.n_surf])}, 1, dC, s);
     if (horseshoe) {
         int64_t rows_tot = 0;
         for (int q = 0; q < L.n_surf; ++q) rows_tot += (int64_t)((L.ms[q] == 0 ? 0 : 1) + 1) * (L.n[q] + 1);
@@ -1269,11 +1313,10 @@ static int run_static(const Plan& p, const fj_case_buffers* B, const double* hg,
     }
     for (int q = 0; q < L.n_surf; ++q) sb.add(p, zb + L.vo[q] * 3, gb + L.po[q], L.m[q], L.n[q]);
     FJ_TRY(pack(p, sb, 0, s));
-    k_force_targets<<<nblk(L.fo[L.n_surf]), 256, 0, s>>>(dC); note_launch();
     FJ_TRY(vind_sum(p, p.targets, L.fo[L.n_surf], sb.len(), sb.n_links, p.v, s));
-    k_force_filament<<<nblk(L.fo[L.n_surf]), 256, 0, s>>>(dC); note_launch();
+    launch_parts(k_filaments, {nblk(L.fo[L.n_surf])}, 1, dC, s);
     k_vertex_forces<<<nblk(L.vo[L.n_surf]), 256, 0, s>>>(dC, 3); note_launch();
-    k_strip_alpha<<<nblk(p.sz_strip), 256, 0, s>>>(dC); note_launch();
+    if (L.any_polar) launch_parts(k_strips, {nblk(p.sz_strip)}, 1, dC, s);
     if (L.any_polar) {  // uvlm.py:1055-1075: forces, then the circulations and the static wake
         k_polar_strips<<<nblk(p.sz_strip), 256, 0, s>>>(dC); note_launch();
         k_polar_vertices<<<nblk(L.vo[L.n_surf]), 256, 0, s>>>(dC); note_launch();
@@ -1283,7 +1326,7 @@ static int run_static(const Plan& p, const fj_case_buffers* B, const double* hg,
         }
     }
     FJ_CUDA(cudaMemsetAsync(B->d_gamma_b_dot, 0, p.sz_pan * sizeof(double), s));
-    k_force_total<<<1, 256, 0, s>>>(dC); note_launch();
+    launch_parts(k_strips, {L.any_polar ? 0 : nblk(p.sz_strip), 1}, 1, dC, s);
     FJ_LAUNCH_CHECK("static solve");
     return FJ_OK;
 }
@@ -1678,31 +1721,28 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
     const StepCase* dC = (const StepCase*)(d_tab + tl.step);
     const dim3 b(256);
 
-    // 1. time, geometry
-    k_time<<<dim3(1, K), 32, 0, s>>>(dC); note_launch();
-    k_geom_vertices<<<dim3(nblk(max_v), K), b, 0, s>>>(dC); note_launch();
-    k_geom_panels<<<dim3(nblk(max_p), K), b, 0, s>>>(dC); note_launch();
+    // 1. geometry, and what follows from it alone
+    const unsigned b_shed = nblk(max_w), b_targets = nblk(max_f);
+    k_vertices<<<dim3(nblk(max_v), K), b, 0, s>>>(dC); note_launch();
+    launch_parts(k_lattice, {nblk(max_p), any_changed ? nblk(max_v * 3) : 0, any_free ? nblk(max_wt) : 0,
+                             any_free ? 0 : b_shed, any_free ? 0 : b_targets}, K, dC, s);
     // 2. free wake, shed + convect
     if (any_free) {
         FJ_TRY(pack_jobs((const PackJob*)(d_tab + tl.pack_free), K, max_e_free, precision, s));
-        k_gather_wake_targets<<<dim3(nblk(max_wt), K), b, 0, s>>>(dC); note_launch();
         FJ_TRY(launch_sum(jf, cf, d_tab + tl.job_free, d_tab + tl.cta_free, precision, kernel, r_cut, s, persistent_sums,
                           tf));
+        launch_parts(k_lattice, {0, 0, 0, b_shed, b_targets}, K, dC, s);
     }
-    k_wake_shed<<<dim3(nblk(max_w), K), b, 0, s>>>(dC); note_launch();
     if (any_var) {  // delta_w surfaces: convect all rows, then re-discretise (aero/utils.py:452-491)
         k_wake_shed_var<<<dim3(nblk(max_xw), K), b, 0, s>>>(dC); note_launch();
         k_wake_redisc_z<<<dim3(nblk(max_cols), K), b, 0, s>>>(dC); note_launch();
         k_wake_redisc_g<<<dim3(nblk(max_cols), K), b, 0, s>>>(dC); note_launch();
     }
     // 3. AIC (mixed: only where the lattice changed since the factorisation)
-    if (any_changed) {
-        k_changed<<<dim3(nblk(max_v * 3), K), b, 0, s>>>(dC); note_launch();
-    }
     FJ_TRY(aic_launch_jobs((const AicArgs*)(d_tab + tl.aic), K, max_n, max_fil, any_mirror, kernel, s));
     // 4. RHS
-    FJ_TRY(pack_jobs((const PackJob*)(d_tab + tl.pack_wake), K, max_e_wake, precision, s));
-    if (!jrn.empty()) FJ_TRY(pack_jobs((const PackJob*)(d_tab + tl.pack_near), K, max_e_near, FJ_PREC_FP64, s));
+    FJ_TRY(pack_jobs((const PackJob*)(d_tab + tl.pack_wake), K, max_e_wake, precision, s,
+                     (const PackJob*)(d_tab + tl.pack_near), jrn.empty() ? 0 : K, max_e_near));
     for (int k = 0; k < K; ++k)  // cases without (far) wake filaments: zero, then the near rows add
         if (rhs_far[k] == 0 && items[k].p.nb > 0)
             FJ_CUDA(cudaMemsetAsync(items[k].p.v, 0, items[k].p.nb * 3 * sizeof(double), s));
@@ -1733,34 +1773,27 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
     }
     // 6. forces with bound(n) + wake(n)
     FJ_TRY(pack_jobs((const PackJob*)(d_tab + tl.pack_bound), K, max_e_bound, precision, s));
-    k_force_targets<<<dim3(nblk(max_f), K), b, 0, s>>>(dC); note_launch();
     FJ_TRY(launch_sum(jfo, cfo, d_tab + tl.job_force, d_tab + tl.cta_force, precision, kernel, r_cut, s, persistent_sums,
                       tfo));
-    k_force_filament<<<dim3(nblk(max_f), K), b, 0, s>>>(dC); note_launch();
     // 7. gamma_dot, vertex forces, strip alpha, totals
+    launch_parts(k_filaments, {b_targets, any_polar ? 0 : nblk(max_n)}, K, dC, s);
+    int64_t max_s = 0;
+    for (const BatchItem& it : items) max_s = std::max(max_s, it.p.sz_strip);
     if (!any_polar) {
-        k_gamma_dot<<<dim3(nblk(max_n), K), b, 0, s>>>(dC); note_launch();
         k_vertex_forces<<<dim3(nblk(max_v), K), b, 0, s>>>(dC, 3); note_launch();
     } else {
         // uvlm.py:1055-1103: steady forces and strip alpha from the solved Gamma, the polar
         // forces and circulation blend, then gamma_dot and the unsteady forces from the
         // blended Gamma (the same kernels; a case without polars skips the polar ones)
-        int64_t max_s = 0;
-        for (const BatchItem& it : items) max_s = std::max(max_s, it.p.sz_strip);
         k_vertex_forces<<<dim3(nblk(max_v), K), b, 0, s>>>(dC, 1); note_launch();
-        k_strip_alpha<<<dim3(nblk(max_s), K), b, 0, s>>>(dC); note_launch();
+        launch_parts(k_strips, {nblk(max_s)}, K, dC, s);
         k_polar_strips<<<dim3(nblk(max_s), K), b, 0, s>>>(dC); note_launch();
         k_polar_vertices<<<dim3(nblk(max_v), K), b, 0, s>>>(dC); note_launch();
         k_polar_gamma<<<dim3(nblk(max_n), K), b, 0, s>>>(dC); note_launch();
-        k_gamma_dot<<<dim3(nblk(max_n), K), b, 0, s>>>(dC); note_launch();
+        launch_parts(k_filaments, {0, nblk(max_n)}, K, dC, s);
         k_vertex_forces<<<dim3(nblk(max_v), K), b, 0, s>>>(dC, 2); note_launch();
     }
-    if (!any_polar) {
-        int64_t max_strip = 0;
-        for (const BatchItem& it : items) max_strip = std::max(max_strip, it.p.sz_strip);
-        k_strip_alpha<<<dim3(nblk(max_strip), K), b, 0, s>>>(dC); note_launch();
-    }
-    k_force_total<<<dim3(1, K), b, 0, s>>>(dC); note_launch();
+    launch_parts(k_strips, {any_polar ? 0 : nblk(max_s), 1}, K, dC, s);
     FJ_LAUNCH_CHECK("step: forces");
     return FJ_OK;
 }

@@ -258,13 +258,16 @@ __global__ void pack32_kernel(PackArgs a, Elem32* __restrict__ out) {
     out[e] = r;
 }
 
-__global__ void pack_jobs_kernel(const PackJob* __restrict__ jobs, int fp64) {
-    const PackJob& J = jobs[blockIdx.y];
+// blockIdx.y: the jobs of the first table, then those of the second (in FP64).
+__global__ void pack_jobs_kernel(const PackJob* __restrict__ jobs, int n_jobs, int fp64,
+                                 const PackJob* __restrict__ jobs64) {
+    const bool second = (int)blockIdx.y >= n_jobs;
+    const PackJob& J = second ? jobs64[blockIdx.y - n_jobs] : jobs[blockIdx.y];
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= J.a.offset[J.a.n_lat]) return;
     PackedLink o;
     pack_one(J.a, e, o);
-    if (fp64) {
+    if (fp64 || second) {
         Elem64 r;
         r.x = o.v[0];
         r.y = o.v[1];
@@ -298,10 +301,13 @@ __global__ void pack_jobs_kernel(const PackJob* __restrict__ jobs, int fp64) {
     }
 }
 
-int pack_jobs(const PackJob* d_jobs, int n_jobs, int64_t max_elem, int precision, cudaStream_t s) {
-    if (n_jobs == 0 || max_elem == 0) return FJ_OK;
-    dim3 g((unsigned)((max_elem + 255) / 256), (unsigned)n_jobs);
-    pack_jobs_kernel<<<g, 256, 0, s>>>(d_jobs, precision == FJ_PREC_FP64); note_launch();
+int pack_jobs(const PackJob* d_jobs, int n_jobs, int64_t max_elem, int precision, cudaStream_t s,
+              const PackJob* d_jobs64, int n_jobs64, int64_t max_elem64) {
+    if (n_jobs == 0 || max_elem == 0) n_jobs = 0, max_elem = 0;
+    if (n_jobs64 == 0 || max_elem64 == 0) n_jobs64 = 0, max_elem64 = 0;
+    if (n_jobs + n_jobs64 == 0) return FJ_OK;
+    dim3 g((unsigned)((std::max(max_elem, max_elem64) + 255) / 256), (unsigned)(n_jobs + n_jobs64));
+    pack_jobs_kernel<<<g, 256, 0, s>>>(d_jobs, n_jobs, precision == FJ_PREC_FP64, d_jobs64); note_launch();
     FJ_LAUNCH_CHECK("pack_jobs_kernel");
     return FJ_OK;
 }

@@ -95,7 +95,8 @@ struct PackJob {
 int vind_launch_jobs(const VindJob* d_jobs, const int64_t* d_cta0, int n_jobs, int64_t total_ctas, double pairs,
                      int precision, int kernel, double r_cut, cudaStream_t s, bool persistent = false,
                      int tile = 0);
-int pack_jobs(const PackJob* d_jobs, int n_jobs, int64_t max_elem, int precision, cudaStream_t s);
+int pack_jobs(const PackJob* d_jobs, int n_jobs, int64_t max_elem, int precision, cudaStream_t s,
+              const PackJob* d_jobs64 = nullptr, int n_jobs64 = 0, int64_t max_elem64 = 0);
 int reduce_jobs(const VindJob* d_jobs, int n_jobs, int64_t max_targets, cudaStream_t s);
 // CTAs of one sum (target tiles x pieces), for building cta0; tile = targets per thread of
 // the FP32 sum (2 or 4; 0 = 2), ignored for FP64.
