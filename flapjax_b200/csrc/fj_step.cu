@@ -2066,10 +2066,13 @@ namespace fj {
 // Captured batched steps, one per batch workspace.  A batch whose launch signature (the
 // grid extents, job counts and out-of-table pointers run_steps reports) equals that of the
 // last capture on its workspace uploads its table and replays the graph; any other batch
-// re-captures (updating the executable graph in place where CUDA allows).  The sum kernels
-// are persistent, so the cases' sizes enter only through the grid maxima.
+// re-captures (updating the executable graph in place where CUDA allows, and only where the
+// factored cases' orders are the same: they decide the cluster sizes of the panels and the
+// solve, and no graph's cluster size is changed in place).  The sum kernels are persistent, so
+// the cases' sizes enter only through the grid maxima.
 struct BatchGraph {
     std::vector<int64_t> sig;
+    std::vector<int> orders;
     cudaGraphExec_t exec = nullptr;
     int64_t kernels = 0;
 };
@@ -2089,6 +2092,14 @@ static int step_batched_graph(std::vector<BatchItem>& v, char* d_tab, size_t tab
         g_bg_replays.fetch_add(1);
         return cuda_status(cudaGraphLaunch(bg.exec, s), "batched step graph launch");
     }
+    std::vector<int> orders;
+    for (const BatchItem& it : v)
+        if (it.p.cfg.precision == FJ_PREC_FP64 || it.refactor) orders.push_back(it.p.nb);
+    if (bg.exec != nullptr && bg.orders != orders) {
+        cudaGraphExecDestroy(bg.exec);
+        bg.exec = nullptr;
+    }
+    bg.orders.swap(orders);
     cudaStream_t cs = nullptr;
     FJ_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
     cudaGraph_t graph = nullptr;
