@@ -1139,30 +1139,7 @@ __global__ void residual64_kernel(const double* __restrict__ A, const double* __
 
 __global__ void rel_resid_kernel(const double* __restrict__ r, const double* __restrict__ b, int n,
                                  double* __restrict__ out) {
-    __shared__ double sr[32], sb[32];
-    double mr = 0.0, mb = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        mr = fmax(mr, fabs(r[i]));
-        mb = fmax(mb, fabs(b[i]));
-        if (r[i] != r[i]) mr = INFINITY;  // NaN propagates as a failure
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        mr = fmax(mr, __shfl_down_sync(0xffffffffu, mr, off));
-        mb = fmax(mb, __shfl_down_sync(0xffffffffu, mb, off));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        sr[threadIdx.x >> 5] = mr;
-        sb[threadIdx.x >> 5] = mb;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-            mr = fmax(mr, sr[w]);
-            mb = fmax(mb, sb[w]);
-        }
-        *out = mb > 0.0 ? mr / mb : mr;
-    }
+    relative_residual(r, b, n, out);
 }
 
 int refine_solve(const double* a, const float* xinv, int n, const double* b, double* x, double* r_buf,
@@ -1200,34 +1177,6 @@ __global__ void residual64_jobs_kernel(const RefineJob* __restrict__ jobs) {
     if (lane == 0) J.r[row] = J.b[row] - acc;
 }
 
-__global__ void rel_resid_jobs_kernel(const RefineJob* __restrict__ jobs) {
-    const RefineJob& J = jobs[blockIdx.x];
-    __shared__ double sr[32], sb[32];
-    double mr = 0.0, mb = 0.0;
-    for (int i = threadIdx.x; i < J.n; i += blockDim.x) {
-        mr = fmax(mr, fabs(J.r[i]));
-        mb = fmax(mb, fabs(J.b[i]));
-        if (J.r[i] != J.r[i]) mr = INFINITY;
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        mr = fmax(mr, __shfl_down_sync(0xffffffffu, mr, off));
-        mb = fmax(mb, __shfl_down_sync(0xffffffffu, mb, off));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        sr[threadIdx.x >> 5] = mr;
-        sb[threadIdx.x >> 5] = mb;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-            mr = fmax(mr, sr[w]);
-            mb = fmax(mb, sb[w]);
-        }
-        *J.resid = mb > 0.0 ? mr / mb : mr;
-    }
-}
-
 int refine_jobs(const RefineJob* d_jobs, int n_jobs, int max_n, int n_iter, cudaStream_t s) {
     if (n_jobs == 0 || max_n == 0) return FJ_OK;
     const int wpb = 8;
@@ -1238,7 +1187,6 @@ int refine_jobs(const RefineJob* d_jobs, int n_jobs, int max_n, int n_iter, cuda
         gemv32_jobs_kernel<<<g, wpb * 32, 0, s>>>(d_jobs, 1, 1); note_launch();
     }
     residual64_jobs_kernel<<<g, wpb * 32, 0, s>>>(d_jobs); note_launch();
-    rel_resid_jobs_kernel<<<n_jobs, 1024, 0, s>>>(d_jobs); note_launch();
     FJ_LAUNCH_CHECK("refine_jobs");
     return FJ_OK;
 }

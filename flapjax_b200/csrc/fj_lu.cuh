@@ -45,8 +45,38 @@ struct RefineJob {
     const double* b;
     double* x;
     double* r;          // n doubles of scratch
-    double* resid;      // 1 double: final relative residual
 };
+// x by n_iter sweeps, and the last one's residual in r (relative_residual makes its size of it).
 int refine_jobs(const RefineJob* d_jobs, int n_jobs, int max_n, int n_iter, cudaStream_t s);
+
+#ifdef __CUDACC__
+// max|r| / max|b| by one CTA.
+__device__ __forceinline__ void relative_residual(const double* r, const double* b, int n, double* out) {
+    __shared__ double sr[32], sb[32];
+    double mr = 0.0, mb = 0.0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        mr = fmax(mr, fabs(r[i]));
+        mb = fmax(mb, fabs(b[i]));
+        if (r[i] != r[i]) mr = INFINITY;  // NaN propagates as a failure
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        mr = fmax(mr, __shfl_down_sync(0xffffffffu, mr, off));
+        mb = fmax(mb, __shfl_down_sync(0xffffffffu, mb, off));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        sr[threadIdx.x >> 5] = mr;
+        sb[threadIdx.x >> 5] = mb;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
+            mr = fmax(mr, sr[w]);
+            mb = fmax(mb, sb[w]);
+        }
+        *out = mb > 0.0 ? mr / mb : mr;
+    }
+}
+#endif
 
 }  // namespace fj

@@ -152,6 +152,9 @@ struct StepCase {
     const double* v_rhs;    // wake velocity at collocation points (null: static solve)
     const double* zeta_ref; // mixed path: lattice of the cached AIC (null: no comparison)
     int* changed;           // mixed path: set to 1 when zb_n differs from zeta_ref
+    const double* resid_r;  // mixed path: the refined solve's residual
+    double* resid;          // and its size (null: no refinement)
+    int* step_ctr;          // replayed steps: advanced by the step's last kernel (else null)
     int* nonfinite;         // lowest slot whose total force is not finite (sentinel: none)
     const double* polars;   // polar tables (Layout::plo blocks; null: no polar correction)
     double* polar_tmp;      // per strip: sectional force (3), couple (3), lift scale
@@ -161,7 +164,7 @@ struct StepCase {
 // The small kernels of a step take 2 to 4 us each, all of it latency (of the table, of the
 // arrays it names, and of the launch), so what may run side by side shares a launch: a kernel
 // of several parts gives each a range of blocks.  A step of an 8 x 32 wing, 34 launches: 148 us
-// (mixed) and 336 us (FP64); these parts together, 27 launches: 129 and 316 us.  Letting each
+// (mixed) and 336 us (FP64); these parts together, 25 launches: 126 and 316 us.  Letting each
 // launch begin while the one before ends (programmatic dependent launch) gave 145 us.
 struct Parts {
     unsigned end[5];  // block after each part's last
@@ -597,11 +600,12 @@ __device__ __forceinline__ void gamma_dot(const StepCase& C, const int64_t p) {
     C.gbd_n[p] = cur * C.relax + C.gbd_nm1[p] * (1.0 - C.relax);
 }
 
-// The filament forces and gamma_dot.
+// The filament forces, gamma_dot and the size of the refined solve's residual.
 __global__ void k_filaments(const StepCase* __restrict__ T, Parts parts) {
     const StepCase& C = T[blockIdx.y];
     if (blockIdx.x < parts.end[0]) force_filament(C, part_index(parts, 0));
-    else gamma_dot(C, part_index(parts, 1));
+    else if (blockIdx.x < parts.end[1]) gamma_dot(C, part_index(parts, 1));
+    else if (C.resid != nullptr) relative_residual(C.resid_r, C.rhs, C.nb, C.resid);
 }
 
 // split_to_vertex of the filament forces (aero/utils.py:220-222) and of
@@ -844,6 +848,7 @@ __global__ void k_strips(const StepCase* __restrict__ T, Parts parts) {
     const StepCase& C = T[blockIdx.y];
     if (blockIdx.x < parts.end[0]) strip_alpha(C, part_index(parts, 0));
     else force_total(C);
+    if (blockIdx.x == parts.end[0] && threadIdx.x == 0 && C.step_ctr != nullptr) *C.step_ctr += 1;
 }
 
 static Parts parts_of(std::initializer_list<unsigned> blocks) {
@@ -1214,10 +1219,6 @@ __global__ void k_select_table(const char* __restrict__ all, size_t stride, cons
         dst[w] = src[w];
 }
 
-__global__ void k_advance(int* ctr) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) *ctr += 1;
-}
-
 // ------------------------------------------------------------------------------------
 // Static solve (uvlm.py:1286-1333 through base_solve_from_grid with static=True)
 // ------------------------------------------------------------------------------------
@@ -1342,6 +1343,7 @@ struct BatchItem {
     const double* hg_n;
     const double* hgd_n;
     const double* hg_nm1;
+    int* step_ctr = nullptr;        // replayed steps: the counter that the step advances
     bool reuse_convection = false;  // free wake: the previous call's convection velocities hold
 };
 
@@ -1424,6 +1426,7 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
         // reused from there when the caller says the step's n-1 state is the same
         const bool fw = c.free_wake && L.wto[L.n_surf] > 0;
         C.free_wake = fw && !it.reuse_convection;
+        C.step_ctr = it.step_ctr;
         C.dt = c.dt;
         C.relax = c.gamma_dot_relaxation;
         C.flow = c.flow;
@@ -1601,7 +1604,8 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
             rj.b = p.rhs;
             rj.x = C.gb_n;
             rj.r = p.r;
-            rj.resid = p.resid + i;
+            C.resid_r = p.r;
+            C.resid = p.resid + i;
             ref.push_back(rj);
         }
     }
@@ -1776,7 +1780,7 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
     FJ_TRY(launch_sum(jfo, cfo, d_tab + tl.job_force, d_tab + tl.cta_force, precision, kernel, r_cut, s, persistent_sums,
                       tfo));
     // 7. gamma_dot, vertex forces, strip alpha, totals
-    launch_parts(k_filaments, {b_targets, any_polar ? 0 : nblk(max_n)}, K, dC, s);
+    launch_parts(k_filaments, {b_targets, any_polar ? 0 : nblk(max_n), ref.empty() ? 0u : 1u}, K, dC, s);
     int64_t max_s = 0;
     for (const BatchItem& it : items) max_s = std::max(max_s, it.p.sz_strip);
     if (!any_polar) {
@@ -1892,10 +1896,11 @@ static int run_range_graph(const Plan& p, const fj_case_buffers* B, int g0, int 
     std::vector<int64_t> sig;
     for (int k = g0; k < g1; ++k) {
         std::vector<BatchItem> one(1, step_item(p, B, k, false));
+        one[0].step_ctr = p.step_ctr;
         FJ_TRY(run_steps(one, p.tab, p.tab_bytes, s, kStepBuild, h.data() + (size_t)(k - g0) * p.tab_bytes,
                          k == g0 ? &sig : nullptr));
     }
-    // the graph's own select and advance kernels take the slot tables, the counter and a
+    // the graph's own select kernel takes the slot tables, the counter and a
     // status word: the counter's place in the workspace follows the slot count, so a
     // workspace at the same address for a case of another length must not replay this graph
     sig.push_back((int64_t)(uintptr_t)p.tab_all);
@@ -1921,7 +1926,6 @@ static int run_range_graph(const Plan& p, const fj_case_buffers* B, int g0, int 
             note_launch();
             std::vector<BatchItem> one(1, step_item(p, B, g0, false));
             st = run_steps(one, p.tab, p.tab_bytes, cs, kStepLaunch);
-            k_advance<<<1, 32, 0, cs>>>(p.step_ctr); note_launch();
             const int st_end = cuda_status(cudaStreamEndCapture(cs, &graph), "step graph capture");
             if (st == FJ_OK) st = st_end;
         }
