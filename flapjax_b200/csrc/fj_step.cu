@@ -1366,7 +1366,7 @@ static void assign_splits(std::vector<VindJob>& jobs, int precision) {
 }
 
 static int launch_sum(const std::vector<VindJob>& jobs, const std::vector<int64_t>& cta0, char* d_jobs, char* d_cta0,
-                      int precision, int kernel, double r_cut, cudaStream_t s, bool persistent, int tile) {
+                      int precision, int kernel, double r_cut, cudaStream_t s, bool replayed, int tile) {
     if (jobs.empty()) return FJ_OK;
     double pairs = 0.0;
     int64_t max_t = 0;
@@ -1375,7 +1375,7 @@ static int launch_sum(const std::vector<VindJob>& jobs, const std::vector<int64_
         max_t = std::max(max_t, j.n_targets);
     }
     FJ_TRY(vind_launch_jobs((const VindJob*)d_jobs, (const int64_t*)d_cta0, (int)jobs.size(), cta0.back(), pairs,
-                            precision, kernel, r_cut, s, persistent, tile));
+                            precision, kernel, r_cut, s, replayed, tile));
     return reduce_jobs((const VindJob*)d_jobs, (int)jobs.size(), max_t, s);
 }
 
@@ -1386,7 +1386,7 @@ enum { kStepNormal = 0, kStepBuild = 1, kStepLaunch = 2 };
 
 static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_bytes, cudaStream_t s,
                      int mode = kStepNormal, char* h_out = nullptr, std::vector<int64_t>* sig = nullptr,
-                     bool persistent_sums = false) {
+                     bool replayed_sums = false) {
     const int K = (int)items.size();
     if (K == 0) return FJ_OK;
     const int precision = items[0].p.cfg.precision;
@@ -1688,19 +1688,20 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
         double rc = r_cut;
         int64_t rc_bits = 0;
         memcpy(&rc_bits, &rc, sizeof(rc_bits));
-        auto sum_sig = [&](const std::vector<VindJob>& jobs) {
+        auto sum_sig = [&](const std::vector<VindJob>& jobs, const std::vector<int64_t>& cta0) {
             int64_t mt = 0;
             for (const VindJob& j : jobs) mt = std::max(mt, j.n_targets);
             g.push_back((int64_t)jobs.size());
             g.push_back(mt);
+            g.push_back(vind_replay_ctas(cta0.back()));
         };
         g = {precision, kernel, rc_bits, K, max_v, max_p, max_w, max_wt, max_f, max_n, max_fil, any_mirror, any_free,
              any_changed, any_var, any_polar, max_xw, max_cols, max_e_free, max_e_wake, max_e_bound, max_e_near,
              (int64_t)ref.size(), tf, tr, tfo};
-        sum_sig(jf);
-        sum_sig(jr);
-        sum_sig(jrn);
-        sum_sig(jfo);
+        sum_sig(jf, cf);
+        sum_sig(jr, cr);
+        sum_sig(jrn, crn);
+        sum_sig(jfo, cfo);
         for (int k = 0; k < K; ++k) {
             const Plan& p = items[k].p;
             g.push_back(p.sz_strip);
@@ -1733,7 +1734,7 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
     // 2. free wake, shed + convect
     if (any_free) {
         FJ_TRY(pack_jobs((const PackJob*)(d_tab + tl.pack_free), K, max_e_free, precision, s));
-        FJ_TRY(launch_sum(jf, cf, d_tab + tl.job_free, d_tab + tl.cta_free, precision, kernel, r_cut, s, persistent_sums,
+        FJ_TRY(launch_sum(jf, cf, d_tab + tl.job_free, d_tab + tl.cta_free, precision, kernel, r_cut, s, replayed_sums,
                           tf));
         launch_parts(k_lattice, {0, 0, 0, b_shed, b_targets}, K, dC, s);
     }
@@ -1750,8 +1751,8 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
     for (int k = 0; k < K; ++k)  // cases without (far) wake filaments: zero, then the near rows add
         if (rhs_far[k] == 0 && items[k].p.nb > 0)
             FJ_CUDA(cudaMemsetAsync(items[k].p.v, 0, items[k].p.nb * 3 * sizeof(double), s));
-    FJ_TRY(launch_sum(jr, cr, d_tab + tl.job_rhs, d_tab + tl.cta_rhs, precision, kernel, r_cut, s, persistent_sums, tr));
-    FJ_TRY(launch_sum(jrn, crn, d_tab + tl.job_near, d_tab + tl.cta_near, FJ_PREC_FP64, kernel, r_cut, s, persistent_sums,
+    FJ_TRY(launch_sum(jr, cr, d_tab + tl.job_rhs, d_tab + tl.cta_rhs, precision, kernel, r_cut, s, replayed_sums, tr));
+    FJ_TRY(launch_sum(jrn, crn, d_tab + tl.job_near, d_tab + tl.cta_near, FJ_PREC_FP64, kernel, r_cut, s, replayed_sums,
                       0));
     k_rhs<<<dim3(nblk(max_n), K), b, 0, s>>>(dC); note_launch();
     FJ_LAUNCH_CHECK("step: geometry, wake, RHS");
@@ -1777,7 +1778,7 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
     }
     // 6. forces with bound(n) + wake(n)
     FJ_TRY(pack_jobs((const PackJob*)(d_tab + tl.pack_bound), K, max_e_bound, precision, s));
-    FJ_TRY(launch_sum(jfo, cfo, d_tab + tl.job_force, d_tab + tl.cta_force, precision, kernel, r_cut, s, persistent_sums,
+    FJ_TRY(launch_sum(jfo, cfo, d_tab + tl.job_force, d_tab + tl.cta_force, precision, kernel, r_cut, s, replayed_sums,
                       tfo));
     // 7. gamma_dot, vertex forces, strip alpha, totals
     launch_parts(k_filaments, {b_targets, any_polar ? 0 : nblk(max_n), ref.empty() ? 0u : 1u}, K, dC, s);
@@ -2072,8 +2073,8 @@ namespace fj {
 // last capture on its workspace uploads its table and replays the graph; any other batch
 // re-captures (updating the executable graph in place where CUDA allows, and only where the
 // factored cases' orders are the same: they decide the cluster sizes of the panels and the
-// solve, and no graph's cluster size is changed in place).  The sum kernels are persistent, so
-// the cases' sizes enter only through the grid maxima.
+// solve, and no graph's cluster size is changed in place).  The sum kernels' grids are rounded
+// up, so the cases' sizes enter only through the maxima.
 struct BatchGraph {
     std::vector<int64_t> sig;
     std::vector<int> orders;

@@ -706,13 +706,13 @@ __device__ __forceinline__ int find_job(const int64_t* __restrict__ cta0, int n_
     return lo;
 }
 
-// The grid walks the virtual CTAs 0 .. cta0[n_jobs]-1 of the job table in strides of its
-// size.  Launched with one CTA per virtual CTA it is the plain tiled sum; launched
-// persistent (a fixed grid: the CTAs the GPU holds at once) the launch does not depend on
-// the jobs' sizes, so one captured launch serves any batch of the same job count.  The
-// persistent form is not the default: its last round of virtual CTAs can fall on a subset
-// of the SMs (9 % slower on the 16 x 128 free-wake step than hardware scheduling, whose
-// last partial wave spreads over every SM).
+// One CTA per (job, tile, piece): the hardware hands them out as others end, so unequal ones
+// even out and a last partial wave spreads over every SM.  A captured launch that is to serve
+// other batches of the same job count has its grid rounded up: the CTAs beyond the table's do
+// nothing, and a grid that turns out too small walks the table in strides (a fixed grid of the CTAs the GPU holds at once, each walking the table in its
+// stride, left SMs idle at the end: 16 wings of 12 x 64 panels and fewer, 537 us a sum for 493).
+constexpr int64_t kReplayCtas = 1024;
+
 template <int KER, int T>
 __global__ void __launch_bounds__(kBlock, MinCtas32<T>::value) vind32_jobs_kernel(const VindJob* __restrict__ jobs,
                                                              const int64_t* __restrict__ cta0, int n_jobs) {
@@ -1000,18 +1000,17 @@ int64_t vind_ctas(int64_t n_targets, int n_part, int precision, int tile) {
     return (n_targets + (int64_t)kBlock * T - 1) / ((int64_t)kBlock * T) * n_part;
 }
 
+int64_t vind_replay_ctas(int64_t total_ctas) { return (total_ctas + kReplayCtas - 1) / kReplayCtas * kReplayCtas; }
+
 int vind_launch_jobs(const VindJob* d_jobs, const int64_t* d_cta0, int n_jobs, int64_t total_ctas, double pairs,
-                     int precision, int kernel, double r_cut, cudaStream_t s, bool persistent, int tile) {
+                     int precision, int kernel, double r_cut, cudaStream_t s, bool replayed, int tile) {
     if (n_jobs == 0 || total_ctas == 0) return FJ_OK;
     if (total_ctas > 0x7fffffff) return fail(FJ_ERR_SHAPE, "vind jobs: grid too large");
     query_occupancy();
-    // one CTA per virtual CTA (the hardware schedules them, and a last partial wave spreads
-    // over every SM), or, persistent, the CTAs the GPU holds at once whatever the jobs need
     const bool wide = precision != FJ_PREC_FP64 && tile == kT32Wide;
     if (precision != FJ_PREC_FP64 && tile != 0 && tile != kT32 && tile != kT32Wide)
         return fail(FJ_ERR_SHAPE, "vind jobs: tile %d (2 or 4 targets per thread)", tile);
-    const int64_t resident = (int64_t)g_sms * (precision == FJ_PREC_FP64 ? g_res64 : (wide ? g_res32w : g_res32));
-    const unsigned g = (unsigned)std::max<int64_t>(1, persistent ? resident : total_ctas);
+    const unsigned g = (unsigned)std::max<int64_t>(1, replayed ? vind_replay_ctas(total_ctas) : total_ctas);
     const int prof = prof_start(s);
     if (precision == FJ_PREC_FP64) {
         const double rc2 = r_cut * r_cut;

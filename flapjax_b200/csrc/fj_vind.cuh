@@ -92,8 +92,10 @@ struct PackJob {
 // Batched launches (one kernel for many jobs; tables in device memory).
 //  vind: CTAs of job j are cta0[j] .. cta0[j+1]-1 (ctas_x(j) * n_split(j) of them);
 //  all jobs of one launch share precision and kernel.
+// CTAs of a captured launch that replays serve with up to as many (`replayed`).
+int64_t vind_replay_ctas(int64_t total_ctas);
 int vind_launch_jobs(const VindJob* d_jobs, const int64_t* d_cta0, int n_jobs, int64_t total_ctas, double pairs,
-                     int precision, int kernel, double r_cut, cudaStream_t s, bool persistent = false,
+                     int precision, int kernel, double r_cut, cudaStream_t s, bool replayed = false,
                      int tile = 0);
 int pack_jobs(const PackJob* d_jobs, int n_jobs, int64_t max_elem, int precision, cudaStream_t s,
               const PackJob* d_jobs64 = nullptr, int n_jobs64 = 0, int64_t max_elem64 = 0);
