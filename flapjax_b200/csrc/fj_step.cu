@@ -141,7 +141,6 @@ struct StepCase {
     double* zb_nm1;         // workspace
     double* c_dot;          // null: no lattice velocity in the RHS (static solve)
     double* targets;
-    double* v;
     double* ffil;
     double* rhs;
     const double* v_wake;   // free-wake convection velocities (null: prescribed wake)
@@ -149,7 +148,10 @@ struct StepCase {
     double* zw_tmp;         // variable wake before re-discretisation (Layout::xvo blocks)
     double* gw_tmp;         // (Layout::xpo blocks)
     double* s_tmp;          // arc length along each wake column (Layout::xvo blocks)
-    const double* v_rhs;    // wake velocity at collocation points (null: static solve)
+    const double* far_part;    // partials of the wake's velocity at the collocation points: all but
+    const double* near_part;   // the near rows', and theirs (none: static solve)
+    const double* force_part;  // and of the velocity at the force targets
+    int n_far, n_near, n_force;
     const double* zeta_ref; // mixed path: lattice of the cached AIC (null: no comparison)
     int* changed;           // mixed path: set to 1 when zb_n differs from zeta_ref
     const double* resid_r;  // mixed path: the refined solve's residual
@@ -164,7 +166,7 @@ struct StepCase {
 // The small kernels of a step take 2 to 4 us each, all of it latency (of the table, of the
 // arrays it names, and of the launch), so what may run side by side shares a launch: a kernel
 // of several parts gives each a range of blocks.  A step of an 8 x 32 wing, 34 launches: 148 us
-// (mixed) and 336 us (FP64); these parts together, 25 launches: 126 and 316 us.  Letting each
+// (mixed) and 336 us (FP64); these parts together, 22 launches: 124 and 316 us.  Letting each
 // launch begin while the one before ends (programmatic dependent launch) gave 145 us.
 struct Parts {
     unsigned end[5];  // block after each part's last
@@ -489,18 +491,74 @@ __device__ __forceinline__ void compare_lattice(const StepCase& C, const int64_t
 // ------------------------------------------------------------------------------------
 // right-hand side (uvlm.py:961-985): b = -((U(c) - c_dot + v_wake) . n)
 // ------------------------------------------------------------------------------------
-__global__ void k_rhs(const StepCase* __restrict__ T) {
+// The sums' partials are added here and in k_filaments, by the kernel that needs the velocities (a
+// launch of its own for it cost 4 us and the way to the next 1).  A CTA of kSumThreads takes
+// 128 / kLanes targets, kLanes threads to each of their three outputs.  Many partials (a case
+// alone) want lanes, whose rounds of loads are the time; few (a case's share of a batch) want
+// targets, since what follows keeps one thread in 3 kLanes: k_rhs of one case with 296
+// partials 8.0 us with 16 lanes, 10.6 with 8, 14.6 with 4; k_filaments of 16 cases with 32
+// each 34.5, 22.0 and 14.4 us.  The choice is by a case's own partials, so that it sums in the same
+// order alone and in a batch.
+constexpr int kSumThreads = 384, kSumMinTargets = 8;
+constexpr int kFewPartials = 40, kSomePartials = 128;  // at most: 4 lanes, 8 lanes
+
+struct SumShared {
+    double part[kSumThreads];
+    double v[kSumThreads / 4];
+};
+
+// S.v = the sums of the CTA's targets over both lists of partials, of n targets each.
+template <int kLanes>
+__device__ __forceinline__ void add_partials(SumShared& S, const double* part0, int n0, const double* part1, int n1,
+                                             int64_t n) {
+    constexpr int kOut = kSumThreads / kLanes;
+    const int o = threadIdx.x % kOut, l = threadIdx.x / kOut;
+    const int64_t i = (int64_t)blockIdx.x * kOut + o;
+    for (int list = 0; list < (n1 > 0 ? 2 : 1); ++list) {
+        const double* part = list ? part1 : part0;
+        const int n_part = list ? n1 : n0;
+        double a = 0.0;
+        if (i < n * 3) {
+#pragma unroll 8
+            for (int k = l; k < n_part; k += kLanes) a += part[(int64_t)k * n * 3 + i];
+        }
+        S.part[threadIdx.x] = a;
+        __syncthreads();
+        if (l == 0) {
+#pragma unroll
+            for (int k = 1; k < kLanes; ++k) a += S.part[k * kOut + o];
+            S.v[o] = list ? S.v[o] + a : a;
+        }
+        __syncthreads();
+    }
+}
+
+// The thread's target with its velocity in v (null: none).
+__device__ __forceinline__ const double* target_sum(SumShared& S, const double* part0, int n0, const double* part1, int n1,
+                                                    int64_t n, int64_t& target) {
+    const int most = max(n0, n1), lanes = most <= kFewPartials ? 4 : most <= kSomePartials ? 8 : 16;
+    const int per = kSumThreads / 3 / lanes;
+    if ((int64_t)blockIdx.x * per >= n) return nullptr;
+    if (lanes == 4) add_partials<4>(S, part0, n0, part1, n1, n);
+    else if (lanes == 8) add_partials<8>(S, part0, n0, part1, n1, n);
+    else add_partials<16>(S, part0, n0, part1, n1, n);
+    target = (int64_t)blockIdx.x * per + threadIdx.x;
+    return (int)threadIdx.x < per && target < n ? S.v + threadIdx.x * 3 : nullptr;
+}
+
+__global__ void __launch_bounds__(kSumThreads) k_rhs(const StepCase* __restrict__ T) {
     const StepCase& C = T[blockIdx.y];
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= C.nb) return;
+    __shared__ SumShared S;
+    int64_t p;
+    const double* v = target_sum(S, C.far_part, C.n_far, C.near_part, C.n_near, C.nb, p);
+    if (v == nullptr) return;
     const double t = C.t[C.i];
     const double x[3] = {C.c[p * 3], C.c[p * 3 + 1], C.c[p * 3 + 2]};
     double u[3];
     flow_eval(C.flow, x, t, u);
     if (C.c_dot != nullptr)
         for (int d = 0; d < 3; ++d) u[d] -= C.c_dot[p * 3 + d];
-    if (C.v_rhs != nullptr)
-        for (int d = 0; d < 3; ++d) u[d] += C.v_rhs[p * 3 + d];
+    for (int d = 0; d < 3; ++d) u[d] += v[d];
     C.rhs[p] = -(u[0] * C.nc[p * 3] + u[1] * C.nc[p * 3 + 1] + u[2] * C.nc[p * 3 + 2]);
 }
 
@@ -554,7 +612,7 @@ __global__ void k_lattice(const StepCase* __restrict__ T, Parts parts) {
     else force_target(C, part_index(parts, 4));
 }
 
-__device__ __forceinline__ void force_filament(const StepCase& C, const int64_t fi) {
+__device__ __forceinline__ void force_filament(const StepCase& C, const int64_t fi, const double* v) {
     const Layout& L = C.L;
     if (fi >= L.fo[L.n_surf]) return;
     const double t = C.t[C.i];
@@ -574,7 +632,7 @@ __device__ __forceinline__ void force_filament(const StepCase& C, const int64_t 
     double vr[3];
     for (int d = 0; d < 3; ++d) {
         const double mpd = 0.5 * (C.zbd_n[ia * 3 + d] + C.zbd_n[ib * 3 + d]);
-        vr[d] = (u[d] + C.v[fi * 3 + d]) - mpd;
+        vr[d] = (u[d] + v[d]) - mpd;
     }
     double g;
     if (chord) {  // gamma_chordwise[:, :-1] = G; gamma_chordwise[:, 1:] += -G
@@ -601,10 +659,14 @@ __device__ __forceinline__ void gamma_dot(const StepCase& C, const int64_t p) {
 }
 
 // The filament forces, gamma_dot and the size of the refined solve's residual.
-__global__ void k_filaments(const StepCase* __restrict__ T, Parts parts) {
+__global__ void __launch_bounds__(kSumThreads) k_filaments(const StepCase* __restrict__ T, Parts parts) {
     const StepCase& C = T[blockIdx.y];
-    if (blockIdx.x < parts.end[0]) force_filament(C, part_index(parts, 0));
-    else if (blockIdx.x < parts.end[1]) gamma_dot(C, part_index(parts, 1));
+    if (blockIdx.x < parts.end[0]) {
+        __shared__ SumShared S;
+        int64_t f;
+        const double* v = target_sum(S, C.force_part, C.n_force, nullptr, 0, C.L.fo[C.L.n_surf], f);
+        if (v != nullptr) force_filament(C, f, v);
+    } else if (blockIdx.x < parts.end[1]) gamma_dot(C, part_index(parts, 1));
     else if (C.resid != nullptr) relative_residual(C.resid_r, C.rhs, C.nb, C.resid);
 }
 
@@ -864,10 +926,10 @@ static inline unsigned nblk(int64_t n, int b = 256) { return (unsigned)((n + b -
 
 // A kernel of several parts over K cases, each part's blocks given.
 static void launch_parts(void (*fn)(const StepCase*, Parts), std::initializer_list<unsigned> blocks, int K,
-                         const StepCase* dC, cudaStream_t s) {
+                         const StepCase* dC, cudaStream_t s, int threads = 256) {
     const Parts p = parts_of(blocks);
     if (p.end[4] == 0) return;
-    fn<<<dim3(p.end[4], (unsigned)K), 256, 0, s>>>(dC, p);
+    fn<<<dim3(p.end[4], (unsigned)K), threads, 0, s>>>(dC, p);
     note_launch();
 }
 
@@ -890,6 +952,8 @@ struct Plan {
     int64_t sz_zb, sz_zw, sz_pan, sz_gw, sz_strip;  // per-slot element counts
     int64_t max_targets, max_stream;
     int64_t part_elems;
+    double* part_near;   // partials of the near rows' sum (mixed)
+    int64_t near_elems;
     size_t ws_needed;    // bytes of workspace this plan carves
     // workspace
     int* flags;          // [0] lu info, [1] geometry changed
@@ -987,6 +1051,8 @@ static TableLayout table_layout(int k) {
     return t;
 }
 
+static int64_t near_splits(int64_t n_elem) { return std::max<int64_t>(1, std::min<int64_t>((n_elem + 31) / 32, 1024)); }
+
 static int make_plan(const fj_case_config* cfg, void* ws, size_t ws_bytes, Plan& p) {
     FJ_TRY(validate(cfg));
     p.cfg = *cfg;
@@ -1027,11 +1093,15 @@ static int make_plan(const fj_case_config* cfg, void* ws, size_t ws_bytes, Plan&
     p.v = a.carve<double>(p.max_targets * 3);
     p.part = a.carve<double>(std::max<int64_t>(part, 1));
     p.stream = a.carve<Elem64>(stream);
+    p.part_near = nullptr;
+    p.near_elems = 0;
     if (cfg->precision == FJ_PREC_MIXED) {
         int64_t near = 0;
         for (int s = 0; s < ns; ++s)
             if (L.ms[s] > 0) near += img * stream_len(std::min(L.ms[s], kNearWakeRows), L.n[s]);
         p.stream_near = a.carve<Elem64>(std::max<int64_t>(near, 1));
+        p.near_elems = std::max(near_splits(near), (int64_t)part_bound(L.po[ns], near, FJ_PREC_FP64)) * L.po[ns] * 3;
+        p.part_near = a.carve<double>(std::max<int64_t>(p.near_elems, 1));
     } else {
         p.stream_near = nullptr;
     }
@@ -1267,7 +1337,8 @@ static int run_static(const Plan& p, const fj_case_buffers* B, const double* hg,
     C.ft = B->d_force_total;
     C.zb_nm1 = p.zeta_nm1;
     C.targets = p.targets;
-    C.v = p.v;
+    C.force_part = p.v;  // one partial: summed by vind_sum
+    C.n_force = 1;
     C.ffil = p.ffil;
     C.rhs = p.rhs;
     C.nonfinite = p.flags + 2;
@@ -1290,7 +1361,7 @@ static int run_static(const Plan& p, const fj_case_buffers* B, const double* hg,
     AicArgs aa;
     fill_aic_args(p, aa, zb, B->d_c, B->d_nc, zw_solve, rows_solve);
     FJ_TRY(aic_launch(aa, nullptr, s));
-    k_rhs<<<nblk(p.nb), 256, 0, s>>>(dC); note_launch();
+    k_rhs<<<nblk(p.nb, kSumMinTargets), kSumThreads, 0, s>>>(dC); note_launch();
     FJ_TRY(lu_factor64(p.a64, p.nb, p.piv, p.flags, s));
     FJ_TRY(lu_solve64(p.a64, p.nb, p.piv, p.rhs, p.r, s));
     FJ_CUDA(cudaMemcpyAsync(gb, p.rhs, p.nb * sizeof(double), cudaMemcpyDeviceToDevice, s));
@@ -1315,7 +1386,7 @@ static int run_static(const Plan& p, const fj_case_buffers* B, const double* hg,
     for (int q = 0; q < L.n_surf; ++q) sb.add(p, zb + L.vo[q] * 3, gb + L.po[q], L.m[q], L.n[q]);
     FJ_TRY(pack(p, sb, 0, s));
     FJ_TRY(vind_sum(p, p.targets, L.fo[L.n_surf], sb.len(), sb.n_links, p.v, s));
-    launch_parts(k_filaments, {nblk(L.fo[L.n_surf])}, 1, dC, s);
+    launch_parts(k_filaments, {nblk(L.fo[L.n_surf], kSumMinTargets)}, 1, dC, s, kSumThreads);
     k_vertex_forces<<<nblk(L.vo[L.n_surf]), 256, 0, s>>>(dC, 3); note_launch();
     if (L.any_polar) launch_parts(k_strips, {nblk(p.sz_strip)}, 1, dC, s);
     if (L.any_polar) {  // uvlm.py:1055-1075: forces, then the circulations and the static wake
@@ -1366,7 +1437,8 @@ static void assign_splits(std::vector<VindJob>& jobs, int precision) {
 }
 
 static int launch_sum(const std::vector<VindJob>& jobs, const std::vector<int64_t>& cta0, char* d_jobs, char* d_cta0,
-                      int precision, int kernel, double r_cut, cudaStream_t s, bool replayed, int tile) {
+                      int precision, int kernel, double r_cut, cudaStream_t s, bool replayed, int tile,
+                      bool reduce = false) {
     if (jobs.empty()) return FJ_OK;
     double pairs = 0.0;
     int64_t max_t = 0;
@@ -1376,7 +1448,7 @@ static int launch_sum(const std::vector<VindJob>& jobs, const std::vector<int64_
     }
     FJ_TRY(vind_launch_jobs((const VindJob*)d_jobs, (const int64_t*)d_cta0, (int)jobs.size(), cta0.back(), pairs,
                             precision, kernel, r_cut, s, replayed, tile));
-    return reduce_jobs((const VindJob*)d_jobs, (int)jobs.size(), max_t, s);
+    return reduce ? reduce_jobs((const VindJob*)d_jobs, (int)jobs.size(), max_t, s) : FJ_OK;
 }
 
 // run_steps modes: build the table and launch (normal); only build the table into a
@@ -1402,7 +1474,7 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
     StepCase* hC = (StepCase*)(h.data() + tl.step);
     std::vector<VindJob> jf, jr, jfo, jrn;
     std::vector<PackJob> pf(K), pw(K), pb(K), pwn(K);
-    std::vector<int64_t> rhs_far(K, 0), near_cap;
+    std::vector<int> far_case, near_case;  // cases of jr's and jrn's jobs
     std::vector<AicArgs> aic(K);
     std::vector<RefineJob> ref;
     std::vector<int> free_idx;
@@ -1457,12 +1529,10 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
         C.zb_nm1 = p.zeta_nm1;
         C.c_dot = p.c_dot;
         C.targets = p.targets;
-        C.v = p.v;
         C.ffil = p.ffil;
         C.rhs = p.rhs;
         C.nonfinite = p.flags + 2;
         C.v_wake = fw ? p.v_conv : nullptr;
-        C.v_rhs = p.v;
         if (L.any_var && B->d_delta_w == nullptr)
             return fail(FJ_ERR_SHAPE, "variable_wake set but d_delta_w is NULL");
         C.delta_w = B->d_delta_w;
@@ -1532,8 +1602,7 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
                            L.ms[q] - kn, L.n[q]);
             }
         }
-        rhs_far[k] = sw.len();
-        const int64_t far_links = sw.n_links;
+        const int64_t far_len = sw.len(), far_links = sw.n_links;
         if (mixed) {
             for (int q = 0; q < L.n_surf; ++q) {
                 const int kn = std::min(L.ms[q], kNearWakeRows);
@@ -1560,11 +1629,13 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
             j.targets = C.c;
             j.n_targets = p.nb;
             j.stream = p.stream;
-            j.n_elem = rhs_far[k];
+            j.n_elem = far_len;
             j.part = p.part;
             j.n_links = far_links;
-            j.out = p.v;
-            if (j.n_elem > 0) jr.push_back(j);
+            if (j.n_elem > 0) {
+                jr.push_back(j);
+                far_case.push_back(k);
+            }
         }
         if (p.nb > 0 && swn.len() > 0) {  // the near rows in FP64, added to the far sum
             VindJob j;
@@ -1573,12 +1644,10 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
             j.n_targets = p.nb;
             j.stream = p.stream_near;
             j.n_elem = swn.len();
-            j.part = p.part;
+            j.part = p.part_near;
             j.n_links = swn.n_links;
-            j.out = p.v;
-            j.accumulate = 1;
             jrn.push_back(j);
-            near_cap.push_back(p.part_elems / ((int64_t)p.nb * 3));
+            near_case.push_back(k);
         }
         {
             VindJob j;
@@ -1589,7 +1658,6 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
             j.n_elem = sw.len() + sbd.len();
             j.part = p.part;
             j.n_links = sw.n_links + sbd.n_links;
-            j.out = p.v;
             jfo.push_back(j);
         }
         // AIC of the bound lattice (dynamic: no wake lumping)
@@ -1614,13 +1682,14 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
     assign_splits(jr, precision);
     assign_splits(jfo, precision);
     // The near-row sums are short (a few rows of links): 32 elements per split so that they
-    // spread over the GPU instead of running as a handful of long FP64 CTAs; each reuses
-    // its case's partial buffer.
-    for (size_t q = 0; q < jrn.size(); ++q)
-        jrn[q].n_split = (int)std::max<int64_t>(1, std::min<int64_t>({(jrn[q].n_elem + 31) / 32, 1024, near_cap[q]}));
+    // spread over the GPU instead of running as a handful of long FP64 CTAs.
+    for (VindJob& j : jrn) j.n_split = (int)near_splits(j.n_elem);
     // every job's partials must fit its case's partial buffer (the kernels take any split)
     std::unordered_map<const double*, int64_t> part_elems;
-    for (const BatchItem& it : items) part_elems[it.p.part] = it.p.part_elems;
+    for (const BatchItem& it : items) {
+        part_elems[it.p.part] = it.p.part_elems;
+        if (it.p.part_near != nullptr) part_elems[it.p.part_near] = it.p.near_elems;
+    }
     for (std::vector<VindJob>* jobs : {&jf, &jr, &jfo, &jrn})
         for (VindJob& j : *jobs) {
             const int64_t cap = part_elems[j.part] / std::max<int64_t>(1, j.n_targets * 3);
@@ -1657,6 +1726,18 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
     cut(jr, precision, tr);
     cut(jfo, precision, tfo);
     cut(jrn, FJ_PREC_FP64, 0);
+    for (size_t q = 0; q < jr.size(); ++q) {
+        hC[far_case[q]].far_part = jr[q].part;
+        hC[far_case[q]].n_far = jr[q].n_split * jr[q].n_sub;
+    }
+    for (size_t q = 0; q < jrn.size(); ++q) {
+        hC[near_case[q]].near_part = jrn[q].part;
+        hC[near_case[q]].n_near = jrn[q].n_split * jrn[q].n_sub;
+    }
+    for (int k = 0; k < K; ++k) {
+        hC[k].force_part = jfo[k].part;
+        hC[k].n_force = jfo[k].n_split * jfo[k].n_sub;
+    }
     auto fill_cta = [&](const std::vector<VindJob>& jobs, size_t off, int prec, int tile) {
         int64_t* c0 = (int64_t*)(h.data() + off);
         c0[0] = 0;
@@ -1705,7 +1786,6 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
         for (int k = 0; k < K; ++k) {
             const Plan& p = items[k].p;
             g.push_back(p.sz_strip);
-            if (rhs_far[k] == 0) g.push_back((int64_t)(uintptr_t)p.v);
             if (precision == FJ_PREC_FP64 || items[k].refactor) {
                 g.push_back(items[k].refactor);
                 for (const void* ptr : {(const void*)p.a64, (const void*)p.piv, (const void*)p.flags,
@@ -1735,7 +1815,7 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
     if (any_free) {
         FJ_TRY(pack_jobs((const PackJob*)(d_tab + tl.pack_free), K, max_e_free, precision, s));
         FJ_TRY(launch_sum(jf, cf, d_tab + tl.job_free, d_tab + tl.cta_free, precision, kernel, r_cut, s, replayed_sums,
-                          tf));
+                          tf, true));
         launch_parts(k_lattice, {0, 0, 0, b_shed, b_targets}, K, dC, s);
     }
     if (any_var) {  // delta_w surfaces: convect all rows, then re-discretise (aero/utils.py:452-491)
@@ -1748,13 +1828,10 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
     // 4. RHS
     FJ_TRY(pack_jobs((const PackJob*)(d_tab + tl.pack_wake), K, max_e_wake, precision, s,
                      (const PackJob*)(d_tab + tl.pack_near), jrn.empty() ? 0 : K, max_e_near));
-    for (int k = 0; k < K; ++k)  // cases without (far) wake filaments: zero, then the near rows add
-        if (rhs_far[k] == 0 && items[k].p.nb > 0)
-            FJ_CUDA(cudaMemsetAsync(items[k].p.v, 0, items[k].p.nb * 3 * sizeof(double), s));
     FJ_TRY(launch_sum(jr, cr, d_tab + tl.job_rhs, d_tab + tl.cta_rhs, precision, kernel, r_cut, s, replayed_sums, tr));
     FJ_TRY(launch_sum(jrn, crn, d_tab + tl.job_near, d_tab + tl.cta_near, FJ_PREC_FP64, kernel, r_cut, s, replayed_sums,
                       0));
-    k_rhs<<<dim3(nblk(max_n), K), b, 0, s>>>(dC); note_launch();
+    k_rhs<<<dim3(nblk(max_n, kSumMinTargets), K), kSumThreads, 0, s>>>(dC); note_launch();
     FJ_LAUNCH_CHECK("step: geometry, wake, RHS");
     // 5. solve
     if (precision == FJ_PREC_FP64) {
@@ -1781,7 +1858,8 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
     FJ_TRY(launch_sum(jfo, cfo, d_tab + tl.job_force, d_tab + tl.cta_force, precision, kernel, r_cut, s, replayed_sums,
                       tfo));
     // 7. gamma_dot, vertex forces, strip alpha, totals
-    launch_parts(k_filaments, {b_targets, any_polar ? 0 : nblk(max_n), ref.empty() ? 0u : 1u}, K, dC, s);
+    launch_parts(k_filaments, {nblk(max_f, kSumMinTargets), any_polar ? 0 : nblk(max_n, kSumThreads), ref.empty() ? 0u : 1u},
+                 K, dC, s, kSumThreads);
     int64_t max_s = 0;
     for (const BatchItem& it : items) max_s = std::max(max_s, it.p.sz_strip);
     if (!any_polar) {
@@ -1795,7 +1873,7 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
         k_polar_strips<<<dim3(nblk(max_s), K), b, 0, s>>>(dC); note_launch();
         k_polar_vertices<<<dim3(nblk(max_v), K), b, 0, s>>>(dC); note_launch();
         k_polar_gamma<<<dim3(nblk(max_n), K), b, 0, s>>>(dC); note_launch();
-        launch_parts(k_filaments, {0, nblk(max_n)}, K, dC, s);
+        launch_parts(k_filaments, {0, nblk(max_n, kSumThreads)}, K, dC, s, kSumThreads);
         k_vertex_forces<<<dim3(nblk(max_v), K), b, 0, s>>>(dC, 2); note_launch();
     }
     launch_parts(k_strips, {any_polar ? 0 : nblk(max_s), 1}, K, dC, s);
