@@ -840,8 +840,8 @@ int split_bound(int64_t n_targets, int64_t n_elem_max, int precision) {
 }
 
 // Partials a sum of up to n_elem_max elements may have (workspace sizing): the splits, or,
-// for few targets, the pieces of one wave of six CTAs on each of 148 SMs.
-constexpr int kPieceWave = 888;
+// for few targets, the pieces of two waves of six CTAs on each of 148 SMs.
+constexpr int kPieceWave = 1776;
 
 int part_bound(int64_t n_targets, int64_t n_elem_max, int precision) {
     const int T = precision == FJ_PREC_FP64 ? kT64 : kT32, fold = precision == FJ_PREC_FP64 ? kFold64 : kFold;
@@ -851,12 +851,14 @@ int part_bound(int64_t n_targets, int64_t n_elem_max, int precision) {
 }
 
 // Pieces per split.  A CTA's time is its links plus a fixed start (targets, first chunk,
-// partials: kStart links' worth).  With few CTAs a sum is latency-bound: the links of a
-// piece run one after the other, so more and shorter pieces win until every SM holds a
-// wave; beyond, whole waves of CTAs take turns on the FP pipe, and a cut only pays where it
-// evens out the last one.  Each extra partial costs the reduction about kReduce links.
-// Measured (8 x 32 wing, 64 wake rows, epsilon kernel, one step's larger sum): FP64 107 us in
-// 19 splits -> 14 us in 304 pieces; FP32 34 -> 8 us.
+// partials: kStart links' worth).  With few CTAs a sum is latency-bound: one on an SM takes as
+// long as two (kAlone) side by side.  Up to a wave the SM that got one more CTA than others ends
+// last, beyond it the hardware hands CTAs out as others end.  Each partial costs the reduction
+// about kReduce links.  Measured (epsilon kernel, the kernel alone, FP32 and FP64 us): 768
+// targets x 12 700 links in 50 splits, 1 to 6, 9 and 17 pieces each: 36, 31, 27, 28, 27, 22, 22, 25
+// and 52, 44, 38, 34, 34, 33, 32, 32; 1612 x 14 500 in 56 splits, 1 to 4: 53, 54, 50, 53 and 81, 80,
+// 75, 77; 8 x 32 wing, 64 wake rows, one step's larger sum in 19 splits alone 34 and 107, in 304
+// pieces 8 and 14.
 int choose_sub(int64_t n_targets, int64_t n_elem, int n_split, int precision, int tile, int64_t max_part) {
     query_occupancy();
     const bool fp64 = precision == FJ_PREC_FP64;
@@ -866,15 +868,14 @@ int choose_sub(int64_t n_targets, int64_t n_elem, int n_split, int precision, in
     const int64_t ctas = (n_targets + (int64_t)kBlock * T - 1) / ((int64_t)kBlock * T) * n_split;
     const int res = fp64 ? g_res64 : (T == kT32Wide ? g_res32w : g_res32);
     const int64_t wave = (int64_t)g_sms * res;
-    constexpr double kStart = 12.0, kReduce = 0.25, kSaturate = 0.75;
+    constexpr double kStart = 4.0, kReduce = 0.1, kAlone = 2.0;
     int best = 1;
     double best_cost = 0.0;
     for (int64_t sub = 1; sub <= max_sub; ++sub) {
         const double len = (double)piece_len(n_elem, n_split, (int)sub, fold) + kStart;
         const int64_t total = ctas * sub;
-        // CTAs one SM runs in turn, its pipes full from kSaturate of its resident CTAs on
-        const double turns = std::max((double)((total + g_sms - 1) / g_sms),
-                                      kSaturate * res * (double)((total + wave - 1) / wave));
+        const double turns = total <= wave ? std::max(kAlone, (double)((total + g_sms - 1) / g_sms))
+                                           : (double)total / g_sms + 0.5;  // (half a CTA: the last ones' tail)
         const double cost = turns * len + kReduce * (double)(n_split * sub);
         if (sub == 1 || cost < 0.98 * best_cost) {
             best = (int)sub;
