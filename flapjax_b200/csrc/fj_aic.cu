@@ -16,10 +16,11 @@
 //     signs, so the sum over rows is the chordwise filaments' plus the first and the last
 //     spanwise one: a quarter of the rings' evaluations.  Every thread takes a stretch of a
 //     chordwise column, whose chain shares its vertices.
-// Assembly with its geometry, epsilon (cutoff) kernel: 12 x 64 rings 20.6 -> 18.6 us (22.7 -> 18.5),
-// 16 x 128 80 -> 63 us (93 -> 66); with the wake's lumping, 8 x 32 + 64 rows 135 -> 16.5 us
-// (160 -> 16.5), 12 x 64 + 120 rows 507 -> 62 us (610 -> 67), against a thread per filament and a
-// thread per strip over all its rings.  One target: 79 (81) us at 16 x 128; four: 79 (81).
+// Assembly with its geometry, epsilon (cutoff) kernel: 12 x 64 rings 20.6 -> 16.5 us (22.7 -> 16.5),
+// 16 x 128 80 -> 60 us (93 -> 61); with the wake's lumping, 8 x 32 + 64 rows 135 -> 16.5 us
+// (160 -> 16.5), 12 x 64 + 120 rows 507 -> 57 us (610 -> 60), against a thread per filament and a
+// thread per strip over all its rings.  At 16 x 128, one target a CTA: 67 (69) us; four: 79 (81);
+// two or four CTAs on an SM for three: 61 (64) and 68 (84).
 #include "fj_aic.cuh"
 #include "fj_bs.cuh"
 
@@ -30,12 +31,14 @@ constexpr int kAicT = 2;  // targets of a CTA
 
 __device__ __forceinline__ void load_vertex(const double* zeta, int64_t v, bool mirrored, const MirrorPlane& mp,
                                             double (&o)[3]) {
-    const double z0 = zeta[v * 3], z1 = zeta[v * 3 + 1], z2 = zeta[v * 3 + 2];
-    const double d0 = z0 - mp.p[0], d1 = z1 - mp.p[1], d2 = z2 - mp.p[2];
-    const double dn = mirrored ? 2.0 * (d0 * mp.nrm[0] + d1 * mp.nrm[1] + d2 * mp.nrm[2]) : 0.0;
-    o[0] = mirrored ? z0 - dn * mp.nrm[0] : z0;
-    o[1] = mirrored ? z1 - dn * mp.nrm[1] : z1;
-    o[2] = mirrored ? z2 - dn * mp.nrm[2] : z2;
+    o[0] = zeta[v * 3];
+    o[1] = zeta[v * 3 + 1];
+    o[2] = zeta[v * 3 + 2];
+    if (mirrored) {
+        const double dn = (o[0] - mp.p[0]) * mp.nrm[0] + (o[1] - mp.p[1]) * mp.nrm[1] + (o[2] - mp.p[2]) * mp.nrm[2];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) o[d] -= 2.0 * dn * mp.nrm[d];
+    }
 }
 
 // The targets of a CTA, their normals over 4 pi (the sums' common factor).
@@ -181,6 +184,8 @@ __device__ __forceinline__ void aic_rows(const AicArgs& a, int64_t i0, double* s
     }
 }
 
+// (Two CTAs on an SM here and three below: with the arguments read from the table three spill, 167 us
+// for 147 on 16 wings.)
 template <int KER, int T>
 __global__ void __launch_bounds__(kAicThreads, 2) aic_jobs_kernel(const AicArgs* __restrict__ tab) {
     const AicArgs& a = tab[blockIdx.y];
@@ -191,7 +196,7 @@ __global__ void __launch_bounds__(kAicThreads, 2) aic_jobs_kernel(const AicArgs*
 }
 
 template <int KER, int T>
-__global__ void __launch_bounds__(kAicThreads, 2) aic_kernel(AicArgs a, const int* __restrict__ run_flag) {
+__global__ void __launch_bounds__(kAicThreads, 3) aic_kernel(AicArgs a, const int* __restrict__ run_flag) {
     if (run_flag != nullptr && *run_flag == 0) return;
     extern __shared__ double sm_inf[];  // [images][T][max filaments], or the wake's partial sums
     aic_rows<KER, T>(a, (int64_t)blockIdx.x * T, sm_inf);
