@@ -1051,7 +1051,9 @@ static TableLayout table_layout(int k) {
     return t;
 }
 
-static int64_t near_splits(int64_t n_elem) { return std::max<int64_t>(1, std::min<int64_t>((n_elem + 31) / 32, 1024)); }
+static int64_t near_splits(int64_t n_elem) {
+    return std::max<int64_t>(1, std::min<int64_t>((n_elem + 31) / 32, 1024));
+}
 
 static int make_plan(const fj_case_config* cfg, void* ws, size_t ws_bytes, Plan& p) {
     FJ_TRY(validate(cfg));
@@ -1913,9 +1915,10 @@ static int check_buffers(const Plan& p, const fj_case_buffers* B, bool dynamic) 
 }
 
 // Status words of a case-level call: flags[0] the LU info of the last factorisation
-// (first zero pivot + 1; the order + 1 where a panel's bounded wait expired), flags[2] the lowest slot with a non-finite total force,
-// flags[3] set when a bounded wait of the tensor-core factorisation expired, flags[4] set
-// when a replayed step graph found its slot counter out of range.
+// (first zero pivot + 1; the order + 1 where a panel's bounded wait expired), flags[2] the
+// lowest slot with a non-finite total force, flags[3] set when a bounded wait of the
+// tensor-core factorisation expired, flags[4] set when a replayed step graph found its slot
+// counter out of range.
 static constexpr int kNoSlot = 0x7f7f7f7f;  // the byte pattern 0x7f repeated
 
 static int clear_status(const Plan& p, cudaStream_t s) {

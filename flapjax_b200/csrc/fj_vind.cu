@@ -709,8 +709,9 @@ __device__ __forceinline__ int find_job(const int64_t* __restrict__ cta0, int n_
 // One CTA per (job, tile, piece): the hardware hands them out as others end, so unequal ones
 // even out and a last partial wave spreads over every SM.  A captured launch that is to serve
 // other batches of the same job count has its grid rounded up: the CTAs beyond the table's do
-// nothing, and a grid that turns out too small walks the table in strides (a fixed grid of the CTAs the GPU holds at once, each walking the table in its
-// stride, left SMs idle at the end: 16 wings of 12 x 64 panels and fewer, 537 us a sum for 493).
+// nothing, and a grid that turns out too small walks the table in strides (a fixed grid of the
+// CTAs the GPU holds at once, each walking the table in its stride, left SMs idle at the end:
+// 16 wings of 12 x 64 panels and fewer, 537 us a sum for 493).
 constexpr int64_t kReplayCtas = 1024;
 
 template <int KER, int T>

@@ -797,7 +797,16 @@ def _steady_force_rows(ops, lay, cfg, Zb, Zw, gb, gw, tZb, tZw, tgb, tgw, lists)
     ncol = lay.n_states + lay.n_inputs
     # filaments of every surface: start, end vertex (global), strength coefficients
     fa, fb, mids, rvec, gval = [], [], [], [], []
-    gcoef = []   # list of (filament, column-in-gamma_b or -1-(gamma_w col), coefficient)
+    # strength coefficients: filament, column in gamma_b or -1 - (column in gamma_w), coefficient.
+    # Lists of numbers, not of tuples: thousands of small objects a call set off the interpreter's
+    # collector (30 ms every tenth call).
+    g_f, g_col, g_co = [], [], []
+
+    def strength(f, col, co):
+        g_f.append(f)
+        g_col.append(col)
+        g_co.append(co)
+
     nf = 0
     for s, (m, n, w) in enumerate(lay.dims):
         z = Zb[s]
@@ -809,9 +818,9 @@ def _steady_force_rows(ops, lay, cfg, Zb, Zw, gb, gw, tZb, tZw, tgb, tgw, lists)
                 fb.append(vb + (k + 1) * (n + 1) + l)
                 g = (G[k, l] if l < n else 0.0) - (G[k, l - 1] if l >= 1 else 0.0)
                 if l < n:
-                    gcoef.append((nf, ob + k * n + l, 1.0))
+                    strength(nf, ob + k * n + l, 1.0)
                 if l >= 1:
-                    gcoef.append((nf, ob + k * n + l - 1, -1.0))
+                    strength(nf, ob + k * n + l - 1, -1.0)
                 gval.append(g)
                 nf += 1
         for k in range(m + 1):      # spanwise (k,l)->(k,l+1), g = G[k-1,l] - G[k,l] (- G_w[0,l] at the TE)
@@ -820,12 +829,12 @@ def _steady_force_rows(ops, lay, cfg, Zb, Zw, gb, gw, tZb, tZw, tgb, tgw, lists)
                 fb.append(vb + k * (n + 1) + l + 1)
                 g = (G[k - 1, l] if k >= 1 else 0.0) - (G[k, l] if k < m else 0.0)
                 if k >= 1:
-                    gcoef.append((nf, ob + (k - 1) * n + l, 1.0))
+                    strength(nf, ob + (k - 1) * n + l, 1.0)
                 if k < m:
-                    gcoef.append((nf, ob + k * n + l, -1.0))
+                    strength(nf, ob + k * n + l, -1.0)
                 if k == m and w > 0:
                     g -= gw[s][0, l]
-                    gcoef.append((nf, -1 - (ow + l), -1.0))
+                    strength(nf, -1 - (ow + l), -1.0)
                 gval.append(g)
                 nf += 1
     fa, fb = np.asarray(fa), np.asarray(fb)
@@ -893,13 +902,11 @@ def _steady_force_rows(ops, lay, cfg, Zb, Zw, gb, gw, tZb, tZw, tgb, tgw, lists)
                 cl.append(zbc[0] + 3 * end + b)
                 vals.append(sign * vx[:, a, b])
     vxr = rho * np.cross(v, rv)                                           # rho (v x r)
-    for f, col, coef in gcoef:
-        colg = gbc[0] + col if col >= 0 else gwc[0] + (-1 - col)
-        for a in range(3):
-            rows.append([3 * f + a])
-            cl.append([colg])
-            vals.append([coef * vxr[f, a]])
-    r_, c_, v_ = (np.concatenate([np.ravel(x) for x in y]) for y in (rows, cl, vals))
+    g_f, g_col = np.asarray(g_f), np.asarray(g_col)
+    rows.append((3 * g_f[:, None] + np.arange(3)).ravel())
+    cl.append(np.repeat(np.where(g_col >= 0, gbc[0] + g_col, (gwc[0] if gwc else 0) - 1 - g_col), 3))
+    vals.append((np.asarray(g_co)[:, None] * vxr[g_f]).ravel())
+    r_, c_, v_ = (np.concatenate(y) for y in (rows, cl, vals))
     df = df.reshape(3 * nf, ncol)
     df.index_put_((torch.as_tensor(r_, device=dev), torch.as_tensor(c_, device=dev)), torch.as_tensor(v_, device=dev),
                   accumulate=True)
