@@ -223,8 +223,8 @@ FJ_API int fj_batch_workspace_size(int max_items, size_t* bytes);
 /* Unless an item has FJ_NO_GRAPH or factorises (no FJ_REUSE_FACTORS), the step runs as a
  * CUDA graph captured on the first call for its batch workspace and replayed by later calls
  * whose batch has the same launch signature: the same number of cases, the same grid
- * maxima and the same sum-job counts (the per-case data travel in the uploaded table; the
- * Biot-Savart sums are persistent kernels whose grid is fixed).  A different signature
+ * maxima and the same sum-job counts and sizes up to a rounding (the per-case data travel
+ * in the uploaded table; the Biot-Savart sums' grids are rounded up).  A different signature
  * re-captures.  Calls that share a batch workspace must not overlap. */
 FJ_API int fj_step_batched(const fj_batch_item* items, int n_items, void* d_batch_ws,
                            size_t batch_ws_bytes, fj_stream_t stream);
