@@ -74,10 +74,11 @@ __device__ __forceinline__ bool outside_core(const double d[3], double r0x, doub
 // |c|^2 > rq = rc2 |r0|^2 with the reference's decision.  The leading words (sign, exponent
 // and 8 mantissa bits) decide where they are not within one of each other; c2's rounding is
 // far below that wherever the pair's velocity matters.  Within one, with no core radius or no
-// length, or where c2 is not finite, `close` is set: the reference's test decides.
+// length, or where c2 is not finite (a NaN of either sign), `close` is set: the reference's test
+// decides, which keeps no NaN.
 __device__ __forceinline__ bool outside_core(double c2, double rq, bool& close) {
     const int hc = __double2hiint(c2) >> 12, hq = __double2hiint(rq) >> 12;
-    close = close || hq == 0 || hc >= 0x7ff00 || (unsigned)(hc - hq + 1) <= 2u;
+    close = close || hq == 0 || (unsigned)hc >= 0x7ff00u || (unsigned)(hc - hq + 1) <= 2u;
     return hc > hq;
 }
 

@@ -1,0 +1,51 @@
+"""FP64 sums whose targets are not numbers: a NaN target keeps no pair of the cutoff kernel (its
+radial distance is not above the radius) and has NaN under the others."""
+from __future__ import annotations
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from flapjax_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+KERNELS = {"epsilon": _lib.FJ_KERNEL_EPSILON, "cutoff": _lib.FJ_KERNEL_CUTOFF, "plain": _lib.FJ_KERNEL_PLAIN}
+NANS = [np.nan, np.array([0xFFF8000000000000], np.uint64).view(float)[0]]  # both signs
+ROWS, COLS, R_CUT = 6, 11, 1e-3
+
+
+def _lattice():
+    rng = np.random.default_rng(4)
+    k, l = np.meshgrid(np.linspace(0, 1, ROWS + 1), np.linspace(0, 2, COLS + 1), indexing="ij")
+    z = np.stack([k + 0.3 * l, l, -0.1 * k], -1)
+    return z, rng.normal(size=(ROWS, COLS)), rng.normal(size=(300, 3)) + [0.5, 1.0, 3.0]
+
+
+def _vind(x, z, g, kernel):
+    import torch
+
+    t, zd, gd = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (x, z, g))
+    rows, cols, v, nb = (C.c_int * 1)(g.shape[0]), (C.c_int * 1)(g.shape[1]), torch.empty_like(t), C.c_size_t()
+    _lib.call("fj_vind_workspace_size", len(x), rows, cols, 1, 0, _lib.FJ_PREC_FP64, C.byref(nb))
+    ws = torch.empty(nb.value, dtype=torch.uint8, device="cuda")
+    p = lambda a: (C.c_void_p * 1)(a.data_ptr())
+    _lib.call("fj_vind", t.data_ptr(), len(x), p(zd), p(gd), rows, cols, 1, None, None, kernel, R_CUT, _lib.FJ_PREC_FP64,
+              v.data_ptr(), ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+    return v.cpu().numpy()
+
+
+@pytest.mark.parametrize("nan", NANS)
+@pytest.mark.parametrize("kernel", ["epsilon", "cutoff", "plain"])
+def test_targets(cuda, kernel, nan):
+    z, g, x = _lattice()
+    want = _vind(x, z, g, KERNELS[kernel])
+    bad = x.copy()
+    bad[3, 1], bad[200] = nan, nan
+    got = _vind(bad, z, g, KERNELS[kernel])
+    others = np.setdiff1d(np.arange(len(x)), [3, 200])
+    assert np.array_equal(got[others], want[others])
+    if kernel == "cutoff":
+        assert np.all(got[[3, 200]] == 0.0)
+    else:
+        assert np.all(np.isnan(got[[3, 200]]))
