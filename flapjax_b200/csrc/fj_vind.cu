@@ -384,18 +384,19 @@ __device__ __forceinline__ void vind64_body(const double* __restrict__ tgt, int6
 
     if (pr.e0 < pr.vend) {
         Vtx64<KER> prev[T];
-        Elem64 pl = st[pr.e0];
-        if (KER == FJ_KERNEL_CUTOFF) pl.q *= rc2;
+        // A link's q as link64 takes it; negative where there is no link: at a chain's last vertex,
+        // and beside a vertex that is not a number.
+        auto staged = [&](Elem64 e) {
+            e.q = e.q >= 0.0 ? (KER == FJ_KERNEL_CUTOFF ? rc2 * e.q : e.q) : -1.0;
+            return e;
+        };
+        Elem64 pl = staged(st[pr.e0]);
 #pragma unroll
         for (int j = 0; j < T; ++j) vtx64<KER>(x[j], pl.x, pl.y, pl.z, prev[j]);
         for (int64_t c0 = pr.e0 + 1; c0 <= pr.vend; c0 += kBlock) {
             const int cnt = (int)min((int64_t)kBlock, pr.vend + 1 - c0);
             __syncthreads();
-            if (threadIdx.x < cnt) {
-                Elem64 e = st[c0 + threadIdx.x];
-                if (KER == FJ_KERNEL_CUTOFF) e.q *= rc2;  // (a break keeps its sign)
-                sh[threadIdx.x] = e;
-            }
+            if (threadIdx.x < cnt) sh[threadIdx.x] = staged(st[c0 + threadIdx.x]);
             __syncthreads();
 #pragma unroll 2
             for (int i = 0; i < cnt; ++i) {
@@ -403,7 +404,7 @@ __device__ __forceinline__ void vind64_body(const double* __restrict__ tgt, int6
                 Vtx64<KER> v[T];
 #pragma unroll
                 for (int j = 0; j < T; ++j) vtx64<KER>(x[j], cur.x, cur.y, cur.z, v[j]);
-                if (__double2hiint(pl.q) >= 0)  // not a chain's last vertex
+                if (__double2hiint(pl.q) >= 0)  // a link
                     link64<KER, T>(prev, v, pl.g, pl.r0x, pl.r0y, pl.r0z, pl.q, rc2, acc);
 #pragma unroll
                 for (int j = 0; j < T; ++j) prev[j] = v[j];

@@ -1,5 +1,6 @@
-"""FP64 sums whose targets are not numbers: a NaN target keeps no pair of the cutoff kernel (its
-radial distance is not above the radius) and has NaN under the others."""
+"""FP64 sums whose targets or vertices are not numbers: a NaN target keeps no pair of the cutoff
+kernel (its radial distance is not above the radius) and has NaN under the others; a filament one
+of whose ends is NaN is left out of the sums."""
 from __future__ import annotations
 
 import ctypes as C
@@ -8,6 +9,7 @@ import numpy as np
 import pytest
 
 from flapjax_b200 import _lib
+from oracle import uvlm_ref as R
 
 pytestmark = pytest.mark.gpu
 KERNELS = {"epsilon": _lib.FJ_KERNEL_EPSILON, "cutoff": _lib.FJ_KERNEL_CUTOFF, "plain": _lib.FJ_KERNEL_PLAIN}
@@ -35,6 +37,20 @@ def _vind(x, z, g, kernel):
     return v.cpu().numpy()
 
 
+def _filaments(g):
+    """(vertex, vertex, strength) of a ring lattice's filaments."""
+    p = np.zeros((ROWS + 2, COLS + 2))
+    p[1:-1, 1:-1] = g
+    out = [((k, l), (k + 1, l), p[k + 1, l + 1] - p[k + 1, l]) for k in range(ROWS) for l in range(COLS + 1)]
+    return out + [((k, l), (k, l + 1), p[k, l + 1] - p[k + 1, l + 1]) for k in range(ROWS + 1) for l in range(COLS)]
+
+
+def _sum(x, z, filaments, kernel):
+    pair = {"epsilon": R.bs_epsilon, "plain": R.bs_plain, "cutoff": lambda *a: R.bs_cutoff(*a, R_CUT)}[kernel]
+    at = lambda v: np.broadcast_to(z[v], x.shape)
+    return sum(g * pair(x, at(a), at(b)) for a, b, g in filaments)
+
+
 @pytest.mark.parametrize("nan", NANS)
 @pytest.mark.parametrize("kernel", ["epsilon", "cutoff", "plain"])
 def test_targets(cuda, kernel, nan):
@@ -49,3 +65,16 @@ def test_targets(cuda, kernel, nan):
         assert np.all(got[[3, 200]] == 0.0)
     else:
         assert np.all(np.isnan(got[[3, 200]]))
+
+
+@pytest.mark.parametrize("nan", NANS)
+@pytest.mark.parametrize("whole", [False, True])
+@pytest.mark.parametrize("kernel", ["epsilon", "cutoff", "plain"])
+def test_vertices(cuda, kernel, whole, nan):
+    z, g, x = _lattice()
+    bad = z.copy()
+    bad[2, 3, 0 if whole else 1:] = nan
+    want = _sum(x, z, [f for f in _filaments(g) if (2, 3) not in f[:2]], kernel)
+    got = _vind(x, bad, g, KERNELS[kernel])
+    # 20 eps |r1||r2| / |c| a pair, of pairs up to 1e3 of the sum, distances of 2 to 5 to filaments of 0.2
+    assert np.all(np.linalg.norm(got - want, axis=1) <= 1e-9 * np.linalg.norm(want, axis=1).max())
