@@ -43,6 +43,12 @@ __device__ __forceinline__ double rcp_normal(double x) {
     return fma(y, fma(e, e, e), y);
 }
 
+// x, or a number near 2^1021 for an infinite x (on the integer pipe): a pair so far away that its
+// |c|^2 overflows adds next to nothing, where 0 (1 / x of infinity) times infinity would be NaN.
+__device__ __forceinline__ double capped(double x) {
+    return __hiloint2double(min(__double2hiint(x), 0x7fcfffff), __double2loint(x));
+}
+
 template <int KER>
 struct Vtx64 {
     double d[3];  // x - y
@@ -106,7 +112,7 @@ __device__ __forceinline__ void link64(const Vtx64<KER> (&a)[T], const Vtx64<KER
             const double s2 = r0x * r2[0] + r0y * r2[1] + r0z * r2[2];
             const double dot = fma(a[j].inv, s1, -(b[j].inv * s2));
             // aero/utils.py:619-623 (epsilon), :637-648 (cutoff)
-            val[j] = (g * dot) * rcp_normal(KER == FJ_KERNEL_EPSILON ? c2 + q : c2);
+            val[j] = (g * dot) * rcp_normal(capped(KER == FJ_KERNEL_EPSILON ? c2 + q : c2));
             if (KER == FJ_KERNEL_CUTOFF) keep[j] = outside_core(c2, q, close);
         }
     }

@@ -1,6 +1,6 @@
-"""FP64 sums whose targets or vertices are not numbers: a NaN target keeps no pair of the cutoff
-kernel (its radial distance is not above the radius) and has NaN under the others; a filament one
-of whose ends is NaN is left out of the sums."""
+"""FP64 sums whose targets or vertices are not numbers, are infinite or far away: a NaN target
+keeps no pair of the cutoff kernel (its radial distance is not above the radius) and has NaN
+under the others; a filament one of whose ends is NaN is left out of the sums."""
 from __future__ import annotations
 
 import ctypes as C
@@ -78,3 +78,11 @@ def test_vertices(cuda, kernel, whole, nan):
     got = _vind(x, bad, g, KERNELS[kernel])
     # 20 eps |r1||r2| / |c| a pair, of pairs up to 1e3 of the sum, distances of 2 to 5 to filaments of 0.2
     assert np.all(np.linalg.norm(got - want, axis=1) <= 1e-9 * np.linalg.norm(want, axis=1).max())
+
+
+@pytest.mark.parametrize("kernel", ["epsilon", "cutoff"])
+def test_far_targets(cuda, kernel):
+    """|r1 x r2|^2 overflows: nothing to add, and nothing that is not a number."""
+    z, g, x = _lattice()
+    x[3], x[200] = [1e100, 2e100, 3e100], [-1e90, 1e90, 0.0]
+    assert np.all(np.abs(_vind(x, z, g, KERNELS[kernel])[[3, 200]]) <= 1e-80)
