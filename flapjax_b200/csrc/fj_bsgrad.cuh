@@ -60,12 +60,14 @@ struct FilGrad {
 };
 
 // What both derivatives take from a pair: g s, g b, w; s1, s2 = r0.r_i / n_i^2; k = s (lam.c).
+// False for a pair within the core radius, which adds nothing: the callers leave it out, since its
+// other factors may be NaN.
 struct PairGrad {
     double gs, gb, s1, s2, w[3], s, k;
 };
 
 template <int KER>
-__device__ __forceinline__ void pair_grad(const VtxGrad<KER>& A, const VtxGrad<KER>& B, const FilGrad& f, double rc2,
+__device__ __forceinline__ bool pair_grad(const VtxGrad<KER>& A, const VtxGrad<KER>& B, const FilGrad& f, double rc2,
                                           const double lam[3], PairGrad& o) {
     static_assert(KER != FJ_KERNEL_PLAIN, "the plain kernel has no adjoint");
     double c[3];
@@ -76,18 +78,14 @@ __device__ __forceinline__ void pair_grad(const VtxGrad<KER>& A, const VtxGrad<K
     const double D = KER == FJ_KERNEL_EPSILON ? c2 + f.q : c2;
     const double num = ahead ? c2 + f.e2 : Z, den = ahead ? Z : 1.0;
     const double inv = rcp_normal(den * D);
-    double a = dot_grad(lam, c, 0.0), b = a * (den * inv);
+    const double a = dot_grad(lam, c, 0.0), b = a * (den * inv);
     o.s = (A.inv + B.inv) * num * inv;
     o.s1 = A.inv2 * dot_grad(f.r0, A.d, 0.0);
     o.s2 = B.inv2 * dot_grad(f.r0, B.d, 0.0);
     if (KER == FJ_KERNEL_CUTOFF) {
         bool close = false, keep = outside_core(c2, f.q, close);
-        if (close) {
-            keep = outside_core(A.d, f.r0[0], f.r0[1], f.r0[2], rc2);
-            if (!keep) a = c[0] = c[1] = c[2] = 0.0;  // (they may be NaN)
-        }
-        o.s = keep ? o.s : 0.0;
-        b = keep ? b : 0.0;
+        if (close) keep = outside_core(A.d, f.r0[0], f.r0[1], f.r0[2], rc2);
+        if (!keep) return false;
     }
     o.k = o.s * a;
     o.gs = f.g * o.s;
@@ -95,6 +93,7 @@ __device__ __forceinline__ void pair_grad(const VtxGrad<KER>& A, const VtxGrad<K
     const double b2 = -2.0 * b;
 #pragma unroll
     for (int k = 0; k < 3; ++k) o.w[k] = fma(b2, c[k], lam[k]);
+    return true;
 }
 
 // acc += g d(lam.K)/dx, the pair's terms added up before (acc may be of the size of 1 / (eps
@@ -103,7 +102,7 @@ template <int KER>
 __device__ __forceinline__ void target_grad(const VtxGrad<KER>& A, const VtxGrad<KER>& B, const FilGrad& f, double rc2,
                                             const double lam[3], double (&acc)[3]) {
     PairGrad p;
-    pair_grad<KER>(A, B, f, rc2, lam, p);
+    if (!pair_grad<KER>(A, B, f, rc2, lam, p)) return;
     const double f1 = p.gb * A.inv, f2 = p.gb * B.inv, h0 = f1 - f2, h1 = f1 * p.s1, h2 = f2 * p.s2;
     double t[3];
     cross_grad(p.w, f.r0, t);
@@ -126,7 +125,7 @@ template <int KER, bool kEnd1 = true, bool kEnd2 = true>
 __device__ __forceinline__ void link_grad(const VtxGrad<KER>& A, const VtxGrad<KER>& B, const FilGrad& f, double rc2,
                                           double e4, const double lam[3], LinkGrad& o) {
     PairGrad p;
-    pair_grad<KER>(A, B, f, rc2, lam, p);
+    if (!pair_grad<KER>(A, B, f, rc2, lam, p)) return;
     const double f1 = p.gb * A.inv, f2 = p.gb * B.inv;
     const double se = KER == FJ_KERNEL_EPSILON ? p.s * e4 : 0.0;
     double t[3];

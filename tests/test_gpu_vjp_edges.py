@@ -1,0 +1,36 @@
+"""The Biot-Savart sum's adjoints where a pair must add nothing: targets that are not numbers under
+the cutoff kernel (within the core radius by the reference's test, as any pair that is dropped,
+whatever the other factors are)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from flapjax_b200 import _lib
+from tests.test_gpu_vjp import _device
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(rows=6, cols=11, n=300):
+    rng = np.random.default_rng(8)
+    k, l = np.meshgrid(np.linspace(0, 1, rows + 1), np.linspace(0, 2, cols + 1), indexing="ij")
+    z, gamma = np.stack([k + 0.3 * l, l, -0.1 * k], -1), rng.normal(size=(rows, cols))
+    x = rng.normal(size=(n, 3)) + [0.5, 1.0, 0.0]
+    x[:, 2] = np.where(x[:, 2] < 0, -0.4, 0.3) + x[:, 2]
+    return z, gamma, x, rng.normal(size=x.shape)
+
+
+@pytest.mark.parametrize("bad", [np.nan, -np.nan, np.inf])
+@pytest.mark.parametrize("r_cut", [0.0, 1e-3])
+def test_targets_that_are_not_numbers(cuda, r_cut, bad):
+    z, gamma, x, lam = _case()
+    rows, none = [3, 200], lam.copy()
+    none[rows] = 0.0  # adds exact zeros
+    want = _device(x, z, gamma, none, _lib.FJ_KERNEL_CUTOFF, r_cut, False)
+    x[3, 1], x[200] = bad, bad
+    lam[rows] = bad
+    got = _device(x, z, gamma, lam, _lib.FJ_KERNEL_CUTOFF, r_cut, False)
+    want[0][rows] = 0.0
+    for g, w in zip(got, want):
+        assert np.array_equal(g, w)
