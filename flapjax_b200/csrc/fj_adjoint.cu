@@ -124,6 +124,8 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjCtas)
     const double r0sq = a.r0x * a.r0x + a.r0y * a.r0y + a.r0z * a.r0z, e4 = 4.0 * kEps * r0sq;
     const FilGrad f = {{a.r0x, a.r0y, a.r0z}, kInv4Pi * a.g, KER == FJ_KERNEL_CUTOFF ? rc2 * a.q : a.q,
                        kEps * kEps * r0sq};
+    // (a filament of no length: a c of nothing but rounding would give its ends a direction)
+    const bool counts = live && r0sq > 0.0;
     LinkGrad l;
     memset(&l, 0, sizeof(l));
     for (int64_t c0 = t0; c0 < t1; c0 += kAdjBlock) {
@@ -137,7 +139,7 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjCtas)
             }
         }
         __syncthreads();
-        if (live) {
+        if (counts) {
 #pragma unroll 2
             for (int i = 0; i < cnt; ++i) {
                 const double x[3] = {sx[i][0], sx[i][1], sx[i][2]};

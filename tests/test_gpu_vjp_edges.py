@@ -1,15 +1,16 @@
 """The Biot-Savart sum's adjoints where a pair must add nothing: targets that are not numbers under
 the cutoff kernel (within the core radius by the reference's test, as any pair that is dropped,
-whatever the other factors are)."""
+whatever the other factors are) and filaments of no length."""
 from __future__ import annotations
 
 import numpy as np
 import pytest
 
 from flapjax_b200 import _lib
-from tests.test_gpu_vjp import _device
+from tests.test_gpu_vjp import EPS, _adjoint, _device, _err, _filaments
 
 pytestmark = pytest.mark.gpu
+KERNELS = {"epsilon": _lib.FJ_KERNEL_EPSILON, "cutoff": _lib.FJ_KERNEL_CUTOFF}
 
 
 def _case(rows=6, cols=11, n=300):
@@ -34,3 +35,17 @@ def test_targets_that_are_not_numbers(cuda, r_cut, bad):
     want[0][rows] = 0.0
     for g, w in zip(got, want):
         assert np.array_equal(g, w)
+
+
+@pytest.mark.parametrize("kernel", ["epsilon", "cutoff"])
+def test_filaments_of_no_length(cuda, kernel):
+    z, gamma, x, lam = _case()
+    z[1] = z[2]
+    f, g = _filaments(*gamma.shape, gamma)
+    zf = z.reshape(-1, 3)
+    some = np.linalg.norm(zf[f[:, 0]] - zf[f[:, 1]], axis=1) > 0
+    want_t, want_z, *_ = _adjoint(x, zf, f[some], g[some], lam, KERNELS[kernel], 1e-3)
+    tb, zb, gb = _device(x, z, gamma, lam, KERNELS[kernel], 1e-3, False)
+    assert _err(tb, want_t) <= 12800 * EPS  # as off the surface in test_gpu_vjp
+    assert _err(zb.reshape(-1, 3), want_z) <= 12800 * EPS
+    assert np.all(np.isfinite(gb))
