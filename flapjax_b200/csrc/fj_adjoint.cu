@@ -154,8 +154,8 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjCtas)
     if (e < n_elem) {
         double* o = part + ((int64_t)split * n_elem + e) * 7;
         for (int k = 0; k < 3; ++k) {
-            o[k] = -fma(l.e1, f.r0[k], l.d1[k]);
-            o[3 + k] = -fma(l.e2, f.r0[k], l.d2[k]);
+            o[k] = l.e1 != 0.0 ? -fma(l.e1, f.r0[k], l.d1[k]) : -l.d1[k];  // (r0 may be infinite)
+            o[3 + k] = l.e2 != 0.0 ? -fma(l.e2, f.r0[k], l.d2[k]) : -l.d2[k];
         }
         o[6] = kInv4Pi * l.k;
     }

@@ -1,6 +1,6 @@
 """The Biot-Savart sum's adjoints where a pair must add nothing: targets that are not numbers under
 the cutoff kernel (within the core radius by the reference's test, as any pair that is dropped,
-whatever the other factors are) and filaments of no length."""
+whatever the other factors are), filaments of no length and with an infinite end."""
 from __future__ import annotations
 
 import numpy as np
@@ -48,4 +48,16 @@ def test_filaments_of_no_length(cuda, kernel):
     tb, zb, gb = _device(x, z, gamma, lam, KERNELS[kernel], 1e-3, False)
     assert _err(tb, want_t) <= 12800 * EPS  # as off the surface in test_gpu_vjp
     assert _err(zb.reshape(-1, 3), want_z) <= 12800 * EPS
+    assert np.all(np.isfinite(gb))
+
+
+@pytest.mark.parametrize("r_cut", [0.0, 1e-3])
+def test_infinite_ends(cuda, r_cut):
+    z, gamma, x, lam = _case()
+    f, g = _filaments(*gamma.shape, gamma)
+    some = ~np.any(f == 2 * 12 + 3, axis=1)
+    want_t, want_z, *_ = _adjoint(x, z.reshape(-1, 3), f[some], g[some], lam, _lib.FJ_KERNEL_CUTOFF, r_cut)
+    z[2, 3, 0] = np.inf
+    tb, zb, gb = _device(x, z, gamma, lam, _lib.FJ_KERNEL_CUTOFF, r_cut, False)
+    assert _err(tb, want_t) <= 12800 * EPS and _err(zb.reshape(-1, 3), want_z) <= 12800 * EPS
     assert np.all(np.isfinite(gb))
