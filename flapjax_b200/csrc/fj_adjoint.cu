@@ -62,15 +62,8 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjCtas)
         Elem64 pl = scaled(st[e0]);
         double pe2 = e2_of(pl);
         vertex(pl, prev);
-        for (int64_t c0 = e0 + 1; c0 <= vend; c0 += kAdjBlock) {
-            const int cnt = (int)min((int64_t)kAdjBlock, vend + 1 - c0);
-            __syncthreads();
-            if (threadIdx.x < cnt) {
-                const Elem64 e = scaled(st[c0 + threadIdx.x]);
-                sh[threadIdx.x] = e;
-                se2[threadIdx.x] = e2_of(e);
-            }
-            __syncthreads();
+        bool far = beyond(x[0], x[1], x[2]) || beyond(pl.x, pl.y, pl.z);
+        auto pairs = [&](int cnt, auto is_far) {
 #pragma unroll 2
             for (int i = 0; i < cnt; ++i) {
                 const Elem64 cur = sh[i];
@@ -83,13 +76,26 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjCtas)
                         for (int k = 0; k < 3; ++k) acc[k] += g1[k] + g2[k];
                     } else {
                         const FilGrad f = {{pl.r0x, pl.r0y, pl.r0z}, pl.g, pl.q, pe2};
-                        target_grad<KER>(prev, v, f, rc2, lm, acc);
+                        target_grad<KER, decltype(is_far)::value>(prev, v, f, rc2, lm, acc);
                     }
                 }
                 prev = v;
                 pl = cur;
                 pe2 = se2[i];
             }
+        };
+        for (int64_t c0 = e0 + 1; c0 <= vend; c0 += kAdjBlock) {
+            const int cnt = (int)min((int64_t)kAdjBlock, vend + 1 - c0);
+            __syncthreads();
+            if (threadIdx.x < cnt) {
+                const Elem64 e = scaled(st[c0 + threadIdx.x]);
+                sh[threadIdx.x] = e;
+                se2[threadIdx.x] = e2_of(e);
+                far = far || beyond(e.x, e.y, e.z);
+            }
+            far = __syncthreads_or(far);
+            if (!kAlone && far) pairs(cnt, std::true_type());
+            else pairs(cnt, std::false_type());
         }
     }
     if (ti < n_t) {
@@ -128,6 +134,18 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjCtas)
     const bool counts = live && r0sq > 0.0;
     LinkGrad l;
     memset(&l, 0, sizeof(l));
+    auto pairs = [&](int cnt, auto is_far) {
+#pragma unroll 2
+        for (int i = 0; i < cnt; ++i) {
+            const double x[3] = {sx[i][0], sx[i][1], sx[i][2]};
+            const double lm[3] = {sx[i][3], sx[i][4], sx[i][5]};
+            VtxGrad<KER> A, B;
+            vtx_grad<KER>(x, a.x, a.y, a.z, A);
+            vtx_grad<KER>(x, b.x, b.y, b.z, B);
+            link_grad<KER, decltype(is_far)::value>(A, B, f, rc2, e4, lm, l);
+        }
+    };
+    bool far = beyond(a.x, a.y, a.z) || beyond(b.x, b.y, b.z);
     for (int64_t c0 = t0; c0 < t1; c0 += kAdjBlock) {
         const int cnt = (int)min((int64_t)kAdjBlock, t1 - c0);
         __syncthreads();
@@ -137,19 +155,11 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjCtas)
                 sx[threadIdx.x][k] = tgt[t * 3 + k];
                 sx[threadIdx.x][3 + k] = lam[t * 3 + k];
             }
+            far = far || beyond(sx[threadIdx.x][0], sx[threadIdx.x][1], sx[threadIdx.x][2]);
         }
-        __syncthreads();
-        if (counts) {
-#pragma unroll 2
-            for (int i = 0; i < cnt; ++i) {
-                const double x[3] = {sx[i][0], sx[i][1], sx[i][2]};
-                const double lm[3] = {sx[i][3], sx[i][4], sx[i][5]};
-                VtxGrad<KER> A, B;
-                vtx_grad<KER>(x, a.x, a.y, a.z, A);
-                vtx_grad<KER>(x, b.x, b.y, b.z, B);
-                link_grad<KER>(A, B, f, rc2, e4, lm, l);
-            }
-        }
+        far = __syncthreads_or(far);
+        if (counts && far) pairs(cnt, std::true_type());
+        else if (counts) pairs(cnt, std::false_type());
     }
     if (e < n_elem) {
         double* o = part + ((int64_t)split * n_elem + e) * 7;

@@ -27,6 +27,13 @@
 
 namespace fj {
 
+// Whether a coordinate is finite and 2^160 or more: where none is, a pair's products stay in range.
+__device__ __forceinline__ bool beyond(double x, double y, double z) {
+    constexpr unsigned kHi = (1023u + 160u) << 20;
+    auto far = [](double v) { return ((unsigned)__double2hiint(v) & 0x7fffffffu) - kHi < 0x7ff00000u - kHi; };
+    return far(x) || far(y) || far(z);
+}
+
 template <int KER>
 struct VtxGrad {
     double d[3], inv, inv2, n;  // x - y; 1 / n, 1 / n^2, n
@@ -66,7 +73,9 @@ struct PairGrad {
     double gs, gb, s1, s2, w[3], s, k;
 };
 
-template <int KER>
+// kFar: den D, of the sixth power of a distance, may leave FP64's range before D and K do: divisions
+// one by one.
+template <int KER, bool kFar>
 __device__ __forceinline__ bool pair_grad(const VtxGrad<KER>& A, const VtxGrad<KER>& B, const FilGrad& f, double rc2,
                                           const double lam[3], PairGrad& o) {
     static_assert(KER != FJ_KERNEL_PLAIN, "the plain kernel has no adjoint");
@@ -77,9 +86,17 @@ __device__ __forceinline__ bool pair_grad(const VtxGrad<KER>& A, const VtxGrad<K
     const bool ahead = __double2hiint(P) > 0;
     const double D = KER == FJ_KERNEL_EPSILON ? c2 + f.q : c2;
     const double num = ahead ? c2 + f.e2 : Z, den = ahead ? Z : 1.0;
-    const double inv = rcp_normal(den * D);
-    const double a = dot_grad(lam, c, 0.0), b = a * (den * inv);
-    o.s = (A.inv + B.inv) * num * inv;
+    const double a = dot_grad(lam, c, 0.0);
+    double b;
+    if (kFar) {
+        const double inv = 1.0 / D;
+        b = a * inv;
+        o.s = D == INFINITY ? 0.0 : (A.inv + B.inv) * (num / den * inv);
+    } else {
+        const double inv = rcp_normal(den * D);
+        b = a * (den * inv);
+        o.s = (A.inv + B.inv) * num * inv;
+    }
     o.s1 = A.inv2 * dot_grad(f.r0, A.d, 0.0);
     o.s2 = B.inv2 * dot_grad(f.r0, B.d, 0.0);
     if (KER == FJ_KERNEL_CUTOFF) {
@@ -98,11 +115,11 @@ __device__ __forceinline__ bool pair_grad(const VtxGrad<KER>& A, const VtxGrad<K
 
 // acc += g d(lam.K)/dx, the pair's terms added up before (acc may be of the size of 1 / (eps
 // |r0|^3), see LinkGrad, and a rounding of that size a pair is enough).
-template <int KER>
+template <int KER, bool kFar>
 __device__ __forceinline__ void target_grad(const VtxGrad<KER>& A, const VtxGrad<KER>& B, const FilGrad& f, double rc2,
                                             const double lam[3], double (&acc)[3]) {
     PairGrad p;
-    if (!pair_grad<KER>(A, B, f, rc2, lam, p)) return;
+    if (!pair_grad<KER, kFar>(A, B, f, rc2, lam, p)) return;
     const double f1 = p.gb * A.inv, f2 = p.gb * B.inv, h0 = f1 - f2, h1 = f1 * p.s1, h2 = f2 * p.s2;
     double t[3];
     cross_grad(p.w, f.r0, t);
@@ -121,28 +138,23 @@ struct LinkGrad {
 };
 
 // e4 = 4 eps |r0|^2 (epsilon kernel).
-template <int KER, bool kEnd1 = true, bool kEnd2 = true>
+template <int KER, bool kFar>
 __device__ __forceinline__ void link_grad(const VtxGrad<KER>& A, const VtxGrad<KER>& B, const FilGrad& f, double rc2,
                                           double e4, const double lam[3], LinkGrad& o) {
     PairGrad p;
-    if (!pair_grad<KER>(A, B, f, rc2, lam, p)) return;
+    if (!pair_grad<KER, kFar>(A, B, f, rc2, lam, p)) return;
     const double f1 = p.gb * A.inv, f2 = p.gb * B.inv;
     const double se = KER == FJ_KERNEL_EPSILON ? p.s * e4 : 0.0;
+    const double h1 = fma(-f1, p.s1, f1), h2 = fma(f2, p.s2, f2);
     double t[3];
-    if (kEnd1) {
-        const double h = fma(-f1, p.s1, f1);
-        cross_grad(B.d, p.w, t);
+    cross_grad(B.d, p.w, t);
 #pragma unroll
-        for (int i = 0; i < 3; ++i) o.d1[i] += fma(p.gs, t[i], fma(h, A.d[i], -f2 * B.d[i]));
-        o.e1 = KER == FJ_KERNEL_EPSILON ? fma(p.gb, A.inv - se, o.e1) : o.e1 + f1;
-    }
-    if (kEnd2) {
-        const double h = fma(f2, p.s2, f2);
-        cross_grad(p.w, A.d, t);
+    for (int i = 0; i < 3; ++i) o.d1[i] += fma(p.gs, t[i], fma(h1, A.d[i], -f2 * B.d[i]));
+    o.e1 = KER == FJ_KERNEL_EPSILON ? fma(p.gb, A.inv - se, o.e1) : o.e1 + f1;
+    cross_grad(p.w, A.d, t);
 #pragma unroll
-        for (int i = 0; i < 3; ++i) o.d2[i] += fma(p.gs, t[i], fma(-f1, A.d[i], h * B.d[i]));
-        o.e2 = KER == FJ_KERNEL_EPSILON ? fma(p.gb, se - B.inv, o.e2) : o.e2 - f2;
-    }
+    for (int i = 0; i < 3; ++i) o.d2[i] += fma(p.gs, t[i], fma(-f1, A.d[i], h2 * B.d[i]));
+    o.e2 = KER == FJ_KERNEL_EPSILON ? fma(p.gb, se - B.inv, o.e2) : o.e2 - f2;
     o.k += p.k;
 }
 

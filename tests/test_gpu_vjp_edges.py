@@ -1,6 +1,7 @@
-"""The Biot-Savart sum's adjoints where a pair must add nothing: targets that are not numbers under
-the cutoff kernel (within the core radius by the reference's test, as any pair that is dropped,
-whatever the other factors are), filaments of no length and with an infinite end."""
+"""The Biot-Savart sum's adjoints where a pair must add nothing, or next to nothing: targets that are
+not numbers under the cutoff kernel (within the core radius by the reference's test, as any pair
+that is dropped, whatever the other factors are), filaments of no length, with an infinite end, and
+targets so far away that the sixth power of their distance overflows."""
 from __future__ import annotations
 
 import numpy as np
@@ -61,3 +62,18 @@ def test_infinite_ends(cuda, r_cut):
     tb, zb, gb = _device(x, z, gamma, lam, _lib.FJ_KERNEL_CUTOFF, r_cut, False)
     assert _err(tb, want_t) <= 12800 * EPS and _err(zb.reshape(-1, 3), want_z) <= 12800 * EPS
     assert np.all(np.isfinite(gb))
+
+
+@pytest.mark.parametrize("far", [1e52, 1e60, 1e80, 1e100])
+@pytest.mark.parametrize("kernel", ["epsilon", "cutoff"])
+def test_far_targets(cuda, kernel, far):
+    z, gamma, x, lam = _case()
+    none = lam.copy()
+    none[[3, 200]] = 0.0
+    want = _device(x, z, gamma, none, KERNELS[kernel], 1e-3, False)
+    x[3], x[200] = [far, 2 * far, 3 * far], [-far, 0.0, 0.0]
+    got = _device(x, z, gamma, lam, KERNELS[kernel], 1e-3, False)
+    assert np.all(np.abs(got[0][[3, 200]]) <= 1e-30)
+    got[0][[3, 200]], want[0][[3, 200]] = 0.0, 0.0
+    for a, b in zip(got, want):  # what they add is far below the last place
+        assert _err(a, b) <= 12800 * EPS
