@@ -60,7 +60,7 @@ struct Shared {
     uint64_t tiles[kMaxBuf];   // an owned block's tiles
     uint64_t ready;            // an owned block has every update
     __align__(16) double x[kRing][kB];
-    double rdiag[kB];
+    double diag[kB];
     int dead;
 };
 
@@ -97,11 +97,19 @@ __device__ __forceinline__ void load_tile(const double* __restrict__ lu, int n, 
     }
 }
 
+// A triangle's diagonal: of ones, or given by its reciprocals; or itself, where one of these would
+// not be a normal number (a division stands in the chain: 64 of them in a block).
+enum Diag { kOnes, kReciprocals, kDivisors };
+
+__device__ __forceinline__ bool has_reciprocal(double d) {
+    return ((unsigned)__double2hiint(d) & 0x7fffffffu) - 0x00100000u < 0x7fd00000u - 0x00100000u;
+}
+
 // Four columns of the block's triangle (kHigh: of its rows 32 ..): lower, ascending from
 // j0 = 4 g, or upper, descending from 4 g + 3.  Their rows' lanes come to hold the solved
-// values (times the diagonal, kUnit or not) by the same operations as every lane's x.
-template <bool kTrans, bool kLower, bool kUnit, bool kHigh>
-__device__ __forceinline__ void solve4(const double* tile, const double* rdiag, double& v0, double& v1, int g, int lane) {
+// values (times the diagonal, unless it is unit) by the same operations as every lane's x.
+template <bool kTrans, bool kLower, Diag kDiag, bool kHigh>
+__device__ __forceinline__ void solve4(const double* tile, const double* diag, double& v0, double& v1, int g, int lane) {
     constexpr unsigned full = 0xffffffffu;
     // M(r, c) lies at tile[r][c], or (kTrans) at tile[c][r]
     auto at = [&](int r, int c) { return kTrans ? tile[c * kPitch + r] : tile[r * kPitch + c]; };
@@ -111,7 +119,8 @@ __device__ __forceinline__ void solve4(const double* tile, const double* rdiag, 
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int j = kLower ? 4 * g + i : 4 * g + 3 - i;
-        if (!kUnit) x[i] *= rdiag[j];
+        if (kDiag == kReciprocals) x[i] *= diag[j];
+        if (kDiag == kDivisors) x[i] /= diag[j];
 #pragma unroll
         for (int h = i + 1; h < 4; ++h)
             x[h] = fma(-at(kLower ? 4 * g + h : 4 * g + 3 - h, j), x[i], x[h]);
@@ -129,24 +138,27 @@ __device__ __forceinline__ void solve4(const double* tile, const double* rdiag, 
     }
 }
 
-// One warp solves the block's triangle on v (rows lane, lane + 32).  rdiag: the diagonal's
-// reciprocals (kUnit: none).
-template <bool kTrans, bool kLower, bool kUnit>
-__device__ __forceinline__ void solve_block(const double* tile, const double* rdiag, double& v0, double& v1, int lane) {
+// One warp solves the block's triangle on v (rows lane, lane + 32).
+template <bool kTrans, bool kLower, Diag kDiag>
+__device__ __forceinline__ void solve_block(const double* tile, const double* diag, double& v0, double& v1, int lane) {
     if (kLower) {
 #pragma unroll 2
-        for (int g = 0; g < 8; ++g) solve4<kTrans, kLower, kUnit, false>(tile, rdiag, v0, v1, g, lane);
+        for (int g = 0; g < 8; ++g) solve4<kTrans, kLower, kDiag, false>(tile, diag, v0, v1, g, lane);
 #pragma unroll 2
-        for (int g = 8; g < 16; ++g) solve4<kTrans, kLower, kUnit, true>(tile, rdiag, v0, v1, g, lane);
+        for (int g = 8; g < 16; ++g) solve4<kTrans, kLower, kDiag, true>(tile, diag, v0, v1, g, lane);
     } else {
 #pragma unroll 2
-        for (int g = 15; g >= 8; --g) solve4<kTrans, kLower, kUnit, true>(tile, rdiag, v0, v1, g, lane);
+        for (int g = 15; g >= 8; --g) solve4<kTrans, kLower, kDiag, true>(tile, diag, v0, v1, g, lane);
 #pragma unroll 2
-        for (int g = 7; g >= 0; --g) solve4<kTrans, kLower, kUnit, false>(tile, rdiag, v0, v1, g, lane);
+        for (int g = 7; g >= 0; --g) solve4<kTrans, kLower, kDiag, false>(tile, diag, v0, v1, g, lane);
     }
-    if (!kUnit) {
-        v0 *= rdiag[lane];
-        v1 *= rdiag[lane + 32];
+    if (kDiag == kReciprocals) {
+        v0 *= diag[lane];
+        v1 *= diag[lane + 32];
+    }
+    if (kDiag == kDivisors) {
+        v0 /= diag[lane];
+        v1 /= diag[lane + 32];
     }
 }
 
@@ -230,23 +242,28 @@ __global__ void __launch_bounds__(kThreads, 1)
             const bool unit = lower != kTrans;  // L is unit lower, U^T is not; U is not, L^T is unit upper
             const double* tile = tiles + (size_t)(k % nbuf) * 2 * kTile;
             wait(S, S.tiles[k % nbuf], k / nbuf);
+            bool divide = false;
             if (!unit) {
+                double d[2];
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int r = lane + 32 * h;
-                    S.rdiag[r] = b * kB + r < n ? 1.0 / tile[r * kPitch + r] : 0.0;
+                    d[h] = b * kB + r < n ? tile[r * kPitch + r] : 1.0;
                 }
+                divide = __any_sync(0xffffffffu, !has_reciprocal(d[0]) || !has_reciprocal(d[1]));
+#pragma unroll
+                for (int h = 0; h < 2; ++h) S.diag[lane + 32 * h] = divide ? d[h] : 1.0 / d[h];
             }
             __syncwarp();
             wait(S, S.ready, k);
             double* yb = y + b / nc * kB;
             double v0 = yb[lane], v1 = yb[lane + 32];
-            if (lower) {
-                if (unit) solve_block<kTrans, true, true>(tile, S.rdiag, v0, v1, lane);
-                else solve_block<kTrans, true, false>(tile, S.rdiag, v0, v1, lane);
+            if (unit) {  // (lower where not transposed, as U is the other way round)
+                solve_block<kTrans, !kTrans, kOnes>(tile, S.diag, v0, v1, lane);
+            } else if (divide) {
+                solve_block<kTrans, kTrans, kDivisors>(tile, S.diag, v0, v1, lane);
             } else {
-                if (unit) solve_block<kTrans, false, true>(tile, S.rdiag, v0, v1, lane);
-                else solve_block<kTrans, false, false>(tile, S.rdiag, v0, v1, lane);
+                solve_block<kTrans, kTrans, kReciprocals>(tile, S.diag, v0, v1, lane);
             }
             yb[lane] = v0;
             yb[lane + 32] = v1;
