@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(kJacBlock) vertex_jacobian_kernel(const double
 __global__ void __launch_bounds__(1024) perm_from_piv_kernel(const int32_t* __restrict__ piv, int n,
                                                              int32_t* __restrict__ perm) {
     extern __shared__ int perm_sm[];
-    __shared__ PermScratch S;
+    __shared__ PermScratch<kPermChunk> S;
     build_perm(piv, n, perm_sm, S);
     for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = perm_sm[i];
 }

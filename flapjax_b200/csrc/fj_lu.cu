@@ -742,7 +742,7 @@ int lu_factor32_tc(float* a, int n, int32_t* piv, int* d_info, int* d_err, float
 __global__ void __launch_bounds__(1024) perm_identity_kernel(const int32_t* __restrict__ piv, int n,
                                                              float* __restrict__ y) {
     extern __shared__ int perm_sm[];
-    __shared__ PermScratch S;
+    __shared__ PermScratch<kPermChunk> S;
     build_perm(piv, n, perm_sm, S);
     for (int i = threadIdx.x; i < n; i += blockDim.x) y[(int64_t)i * n + perm_sm[i]] = 1.0f;
 }

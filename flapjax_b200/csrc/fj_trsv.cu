@@ -392,11 +392,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     cl.sync();  // no CTA leaves while another may still send to it
 }
 
+template <int kChunk>
 __global__ void __launch_bounds__(1024) permute_kernel(const int32_t* __restrict__ piv, int n,
                                                        const double* __restrict__ b, double* __restrict__ x,
                                                        int scatter) {
     extern __shared__ int perm[];
-    __shared__ PermScratch S;
+    __shared__ PermScratch<kChunk> S;
     build_perm(piv, n, perm, S);
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         if (scatter) x[perm[i]] = b[i];
@@ -409,7 +410,9 @@ __global__ void __launch_bounds__(1024) permute_kernel(const int32_t* __restrict
 int lu_substitute64(const double* lu, int n, const int32_t* piv, double* b, double* work, bool transposed,
                     cudaStream_t s) {
     const size_t psm = (size_t)n * sizeof(int);
-    FJ_TRY(allow_dynamic_smem((const void*)permute_kernel, psm));
+    if (n > kPermRows<kPermChunkSmall>) return fail(FJ_ERR_UNSUPPORTED, "lu_solve: n=%d too large", n);
+    auto* permute = n <= kPermRows<kPermChunk> ? permute_kernel<kPermChunk> : permute_kernel<kPermChunkSmall>;
+    FJ_TRY(allow_dynamic_smem((const void*)permute, psm));
     const int nb = (n + kB - 1) / kB;
     // one CTA per four blocks: below, the exchange costs more than the reading it shares
     const int nc = std::max(1, std::min(kMaxCtas, nb / 4));
@@ -421,7 +424,7 @@ int lu_substitute64(const double* lu, int n, const int32_t* piv, double* b, doub
     const void* fn = transposed ? (const void*)substitute_kernel<true> : (const void*)substitute_kernel<false>;
     FJ_TRY(allow_dynamic_smem(fn, bytes(nbuf)));
     if (!transposed) {
-        permute_kernel<<<1, 1024, psm, s>>>(piv, n, b, work, 0);
+        permute<<<1, 1024, psm, s>>>(piv, n, b, work, 0);
         note_launch();
     }
     cudaLaunchConfig_t cfg = {};
@@ -438,7 +441,7 @@ int lu_substitute64(const double* lu, int n, const int32_t* piv, double* b, doub
         FJ_CUDA(cudaLaunchKernelEx(&cfg, substitute_kernel<false>, lu, n, (const double*)work, b, nbuf));
     } else {
         FJ_CUDA(cudaLaunchKernelEx(&cfg, substitute_kernel<true>, lu, n, (const double*)b, work, nbuf));
-        permute_kernel<<<1, 1024, psm, s>>>(piv, n, work, b, 1);
+        permute<<<1, 1024, psm, s>>>(piv, n, work, b, 1);
         note_launch();
     }
     note_launch();

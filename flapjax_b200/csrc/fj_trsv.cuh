@@ -10,17 +10,24 @@ namespace fj {
 // in order, bring to row i.  Every thread of the CTA calls it.  Blocks of 64 swaps are
 // composed side by side, a thread tracing one row back through its block, and then applied
 // one after the other: one thread's walk through all swaps took 11 us for 256 and 80 us for
-// 2048.
-constexpr int kPermChunk = 2048;
+// 2048.  kChunk swaps at a time: kPermChunk, or fewer where the scratch has to make room for perm.
+// perm may lie in global memory.
+constexpr int kPermChunk = 2048, kPermChunkSmall = 512;
+template <int kChunk>
 struct PermScratch {
-    int p[kPermChunk], src[2 * kPermChunk];
+    int p[kChunk], src[2 * kChunk];
 };
 
-__device__ __forceinline__ void build_perm(const int32_t* __restrict__ piv, int n, int* perm, PermScratch& S) {
+// The orders whose perm fits in shared memory beside its scratch.
+template <int kChunk>
+constexpr int kPermRows = (232448 - (int)sizeof(PermScratch<kChunk>)) / (int)sizeof(int);
+
+template <int kChunk>
+__device__ __forceinline__ void build_perm(const int32_t* __restrict__ piv, int n, int* perm, PermScratch<kChunk>& S) {
     const int t = threadIdx.x, nt = blockDim.x;
     for (int i = t; i < n; i += nt) perm[i] = i;
-    for (int c0 = 0; c0 < n; c0 += kPermChunk) {
-        const int cnt = min(kPermChunk, n - c0);
+    for (int c0 = 0; c0 < n; c0 += kChunk) {
+        const int cnt = min(kChunk, n - c0);
         __syncthreads();
         for (int i = t; i < cnt; i += nt) S.p[i] = min(max(piv[c0 + i], 0), n - 1);
         __syncthreads();
