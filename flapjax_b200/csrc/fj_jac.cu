@@ -199,13 +199,15 @@ __global__ void __launch_bounds__(kJacBlock) vertex_jacobian_kernel(const double
     }
 }
 
-// perm = the getrf row swaps of piv applied in order to the identity
-__global__ void __launch_bounds__(1024) perm_from_piv_kernel(const int32_t* __restrict__ piv, int n,
-                                                             int32_t* __restrict__ perm) {
+// perm = the getrf row swaps of piv applied in order to the identity (in place where it does
+// not fit in shared memory)
+template <bool kShared>
+__global__ void __launch_bounds__(1024) perm_from_piv_kernel(const int32_t* __restrict__ piv, int n, int32_t* perm) {
     extern __shared__ int perm_sm[];
     __shared__ PermScratch<kPermChunk> S;
-    build_perm(piv, n, perm_sm, S);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = perm_sm[i];
+    build_perm(piv, n, kShared ? perm_sm : perm, S);
+    if (kShared)
+        for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = perm_sm[i];
 }
 
 // Blocked substitution for many right-hand sides.  CTA = 256 threads on a tile of 32
@@ -443,8 +445,11 @@ int fj_lu_solve_many(const double* d_lu, int n, const int32_t* d_piv, double* d_
     char* base = (char*)(((uintptr_t)d_ws + 255) / 256 * 256);
     int32_t* perm = (int32_t*)base;
     double* w = (double*)(base + ((size_t)n * sizeof(int32_t) + 255) / 256 * 256);
-    FJ_TRY(allow_dynamic_smem((const void*)perm_from_piv_kernel, (size_t)n * sizeof(int)));
-    perm_from_piv_kernel<<<1, 1024, (size_t)n * sizeof(int), s>>>(d_piv, n, perm);
+    const bool fits = n <= kPermRows<kPermChunk>;
+    auto* from_piv = fits ? perm_from_piv_kernel<true> : perm_from_piv_kernel<false>;
+    const size_t psm = fits ? (size_t)n * sizeof(int) : 0;
+    FJ_TRY(allow_dynamic_smem((const void*)from_piv, psm));
+    from_piv<<<1, 1024, psm, s>>>(d_piv, n, perm);
     lu_solve_many_kernel<<<(unsigned)((nrhs + kSolveCols - 1) / kSolveCols), kSolveThreads, 0, s>>>(d_lu, n, perm, d_b,
                                                                                              nrhs, ldb, w);
     note_launch(2);

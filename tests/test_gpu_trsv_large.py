@@ -1,6 +1,6 @@
-"""getrs of orders whose row permutation needs a smaller scratch in shared memory (from 51 969),
-and those whose tiles have two buffers (from 17 400): factors of the unit matrix with a few entries
-beside it, and pivots at random."""
+"""getrs of orders whose row permutation needs a smaller scratch in shared memory (from 51 969), or
+does not fit there (many right-hand sides), and those whose tiles have two buffers (from 17 400):
+factors of the unit matrix with a few entries beside it, and pivots at random."""
 from __future__ import annotations
 
 import ctypes as C
@@ -62,3 +62,17 @@ def test_one_right_hand_side(cuda, n):
         _lib.call("fj_lu_solve_t" if transposed else "fj_lu_solve", lu.data_ptr(), n, piv.data_ptr(), x.data_ptr(),
                   ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
         assert np.array_equal(x.cpu().numpy(), _solve(entries, perm, b, transposed))
+
+
+def test_many_right_hand_sides(cuda):
+    import torch
+
+    n = 51969
+    lu, piv, perm, b, entries = _case(torch, n)
+    x, nb = torch.from_numpy(np.stack([b, -2.0 * b], 1).copy()).cuda(), C.c_size_t()
+    _lib.call("fj_lu_solve_many_workspace_size", n, 2, C.byref(nb))
+    ws = torch.zeros(nb.value, dtype=torch.uint8, device="cuda")
+    _lib.call("fj_lu_solve_many", lu.data_ptr(), n, piv.data_ptr(), x.data_ptr(), 2, 2, ws.data_ptr(), ws.numel(),
+              torch.cuda.current_stream().cuda_stream)
+    want = _solve(entries, perm, b, False)
+    assert np.array_equal(x.cpu().numpy(), np.stack([want, -2.0 * want], 1))
