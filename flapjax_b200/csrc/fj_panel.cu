@@ -30,6 +30,7 @@
 // lane and warps: 4 x 1, 2 x 2 and 1 x 8 were slower for one CTA, 256-row CTAs of a cluster up
 // to 12 %.
 #include <climits>
+#include <map>
 #include <mutex>
 
 #include <cooperative_groups.h>
@@ -584,38 +585,43 @@ cudaLaunchConfig_t cluster_config(unsigned ctas, cudaLaunchAttribute* at) {
     return cfg;
 }
 
-// The forms' limits, set once; the rows they take.
+// The rows the forms take on the current device, whose limits this sets (a kernel's attributes
+// belong to a device).
+template <typename T>
+int limits_of_device() {
+    for (int f = 0; f < 4; ++f)
+        if (allow_dynamic_smem((const void*)form<T>(f), (size_t)tile_bytes<T>(f)) != FJ_OK) {
+            cudaGetLastError();
+            return 0;
+        }
+    const Kernel<T> many = form<T>(kCluster);
+    const bool any_size =
+        cudaFuncSetAttribute((const void*)many, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    cudaGetLastError();
+    for (unsigned size : {(unsigned)kMaxCtas, 8u, 4u}) {
+        if (size > 8 && !any_size) continue;
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t cfg = cluster_config<T>(size, &at);
+        int clusters = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, many, &cfg);
+        cudaGetLastError();
+        if (e == cudaSuccess && clusters > 0) return (int)size * form_rows(kCluster);
+    }
+    return form_rows(2);
+}
+
 template <typename T>
 int set_up() {
-    static std::once_flag once;
-    static int rows = 0;
-    std::call_once(once, [] {
-        for (int f = 0; f < 4; ++f) {
-            if (cudaFuncSetAttribute((const void*)form<T>(f), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     tile_bytes<T>(f)) != cudaSuccess) {
-                cudaGetLastError();
-                return;
-            }
-        }
-        const Kernel<T> many = form<T>(kCluster);
-        const bool any_size =
-            cudaFuncSetAttribute((const void*)many, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    static std::mutex mu;
+    static std::map<int, int> rows;  // by device
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
         cudaGetLastError();
-        rows = form_rows(2);
-        for (unsigned size : {(unsigned)kMaxCtas, 8u, 4u}) {
-            if (size > 8 && !any_size) continue;
-            cudaLaunchAttribute at;
-            const cudaLaunchConfig_t cfg = cluster_config<T>(size, &at);
-            int clusters = 0;
-            const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, many, &cfg);
-            cudaGetLastError();
-            if (e == cudaSuccess && clusters > 0) {
-                rows = (int)size * form_rows(kCluster);
-                return;
-            }
-        }
-    });
-    return rows;
+        return 0;
+    }
+    std::lock_guard<std::mutex> g(mu);
+    const auto it = rows.find(dev);
+    return it != rows.end() ? it->second : rows[dev] = limits_of_device<T>();
 }
 
 }  // namespace
