@@ -37,6 +37,13 @@ bool prof_active();
 // kernel on different streams never lower each other's limit between set and launch.
 int allow_dynamic_smem(const void* func, size_t bytes);
 
+// Limit of a wait on an mbarrier, about a second at the B200 SM clock (a test's build sets a
+// negative one, with which every wait expires).
+#ifndef FJ_WAIT_CYCLES
+#define FJ_WAIT_CYCLES 2000000000ll
+#endif
+constexpr long long kSettleCycles = 400000;  // after an expired wait, for the CTA's own sends to arrive
+
 // Opt-in timing of the Biot-Savart sum kernels with CUDA events on their stream
 // (fj_profile_begin / fj_profile_end).  prof_start returns -1 when profiling is off.
 int prof_start(cudaStream_t s);

@@ -144,7 +144,7 @@ __device__ __forceinline__ uint32_t in_cta(uint32_t addr, int rank) {
     return r;
 }
 
-constexpr long long kWaitCycles = 2000000000ll;  // ~1 s at the B200 SM clock
+constexpr long long kWaitCycles = FJ_WAIT_CYCLES;
 
 __device__ __forceinline__ bool try_phase(uint32_t bar, uint32_t parity) {
     uint32_t done;
@@ -158,8 +158,11 @@ __device__ __forceinline__ bool try_phase(uint32_t bar, uint32_t parity) {
     return done != 0;
 }
 
-// Waits for the phase, about a second at most (far beyond any column); false on expiry.
+// Waits for the phase, about a second at most (far beyond any column); false on expiry.  From then on
+// the CTA waits for nothing and expects nothing, works on whatever its slots hold (places and
+// positions in range, since the slots begin with zeros), and writes none of its rows back.
 __device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity) {
+    if (kWaitCycles < 0) return false;
     if (try_phase(bar, parity)) return true;
     const long long t0 = clock64();
     while (!try_phase(bar, parity))
@@ -285,6 +288,7 @@ __device__ __forceinline__ void columns(T (&v)[RPL][kWin<T>], Rows<RPL>& row, T*
 #pragma unroll 1
     for (int j = j0; j < j1; ++j) {
         const int par = j & 1;
+        const bool dead = kCluster && *(volatile int*)&S.dead;
         T x[RPL];
 #pragma unroll
         for (int e = 0; e < RPL; ++e) x[e] = v[e][0];
@@ -314,8 +318,8 @@ __device__ __forceinline__ void columns(T (&v)[RPL][kWin<T>], Rows<RPL>& row, T*
         }
         const Cand<T>* p = &mine;
         if (kCluster) {
-            if (tid == 0) expect_bytes(smem_addr(&S.bar[par]), nc * (int)sizeof(Cand<T>));
-            if (!*(volatile int*)&S.dead && !wait_phase(smem_addr(&S.bar[par]), (j >> 1) & 1)) S.dead = 1;
+            if (tid == 0 && !dead) expect_bytes(smem_addr(&S.bar[par]), nc * (int)sizeof(Cand<T>));
+            if (!dead && !wait_phase(smem_addr(&S.bar[par]), (j >> 1) & 1)) S.dead = 1;
             const uint4 h = *reinterpret_cast<const uint4*>(&S.slot[par][lane & (kMaxCtas - 1)].hi);
             const int o = best_lane({lane < nc ? h.x : 0u, h.y}, lane < nc ? (int)h.z : INT_MAX, lane) & (kMaxCtas - 1);
             p = &S.slot[par][o];
@@ -454,6 +458,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int c = lane; c < KB; c += 32) tile[c * LD + r] = (r0 + r < rows && c < kb) ? src[c] : T(0);
     }
     if (tid < KW) S.zeros[tid] = T(0);
+    if (kCluster && tid < 2 * kMaxCtas)
+        *reinterpret_cast<uint4*>(&S.slot[tid / kMaxCtas][tid % kMaxCtas].hi) = make_uint4(0u, 0u, 0u, 0u);
     if (tid == 0) {
         S.info = INT_MAX;
         S.dead = 0;
@@ -477,7 +483,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int s0 = 0; s0 < kb; s0 += KW) {
         const int end = min(kb, s0 + KW);
         const bool more = end < kb;
-        if (kCluster && more && tid == kThreads - 1) expect_bytes(smem_addr(&S.ubar), KW * KB * (int)sizeof(T));
+        if (kCluster && more && tid == kThreads - 1 && !S.dead) expect_bytes(smem_addr(&S.ubar), KW * KB * (int)sizeof(T));
         if (warp < CW) {
             __align__(16) T v[RPL][KW];
 #pragma unroll
@@ -493,7 +499,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // the pivots, and the pivot rows' windows to their places
         if (tid < end - s0) {
             const Cand<T>& c = S.chosen[tid];
-            S.piv[s0 + tid] = k + c.pos;
+            S.piv[s0 + tid] = k + max(c.pos, 0);  // (-1: a CTA without rows, after an expired wait)
             S.owner[tid] = !kCluster || S.cta[tid] == q ? c.idx : -1;
             if (c.row[0] == T(0)) atomicMin(&S.info, s0 + tid);
         }
@@ -533,21 +539,30 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
         for (int f = 0; f < RPL; ++f) S.pos[base + 32 * f] = row.pos[f];
     __syncthreads();
+    const bool dead = kCluster && S.dead != 0;
 #pragma unroll 4
     for (int r = warp; r < NR; r += kWarps) {
         const int pos = S.pos[r];
-        if (pos < 0) continue;
+        if (pos < 0 || dead) continue;
         T* dst = a + (int64_t)(k + pos) * n + k;
 #pragma unroll
         for (int c = lane; c < KB; c += 32)
             if (c < kb) dst[c] = tile[c * LD + r];
     }
-    if (q == 0) {
-        for (int j = tid; j < kb; j += kThreads) piv[k + j] = S.piv[j];
-        if (tid == 0 && S.info != INT_MAX && *info == 0) *info = k + S.info + 1;
+    if (q == 0)
+        for (int j = tid; j < kb; j += kThreads) piv[k + j] = dead ? k + j : S.piv[j];
+    if (tid == 0) {
+        if (q == 0 && S.info != INT_MAX) atomicCAS(info, 0, k + S.info + 1);
+        if (dead) atomicMax(info, n + 1);  // above any column's
     }
-    if (S.dead && tid == 0) *info = n + 1;
-    if (kCluster) cg::this_cluster().sync();  // no CTA leaves while another may still send to it
+    if (kCluster) {
+        if (dead) {
+            const long long t0 = clock64();
+            while (clock64() - t0 < kSettleCycles) {
+            }
+        }
+        cg::this_cluster().sync();  // no CTA leaves while another may still send to it
+    }
 }
 
 // The forms: column warps and rows per lane for panels of up to 128, 256 and 384 rows in one
