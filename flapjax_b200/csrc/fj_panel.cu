@@ -562,6 +562,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
         }
         cg::this_cluster().sync();  // no CTA leaves while another may still send to it
+        if (dead && tid == 0) a[(int64_t)k * n + k] = (T)NAN;  // so that no solution comes of the factors
     }
 }
 

@@ -346,7 +346,7 @@ FJ_API int fj_aic_workspace_size(const int* m, const int* n, int n_surf, size_t*
 /* jnp.linalg.solve (aero/uvlm.py:985) split as LAPACK getrf/getrs, row-major A.
  * fj_lu_factor overwrites d_a with L\U and writes 0-based pivot rows to d_piv (n).  The
  * workspace's first int32 receives 0, 1 + the column of the first zero pivot, or n + 1 where
- * a bounded wait between the kernel's CTAs expired (the factors are then of no use). */
+ * a bounded wait between a kernel's CTAs expired (a pivot is then NaN). */
 FJ_API int fj_lu_workspace_size(int n, size_t* bytes);
 FJ_API int fj_lu_factor(double* d_a, int n, int32_t* d_piv, void* d_ws, size_t ws_bytes,
                  fj_stream_t stream);

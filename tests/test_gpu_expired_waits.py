@@ -1,5 +1,5 @@
 """A cluster's waits that expire: a build of the kernels in which every wait gives up at once.  The
-panel writes no row, names each row as its own pivot and reports the order + 1."""
+panel writes no row, names each row as its own pivot, reports the order + 1 and leaves a NaN pivot."""
 from __future__ import annotations
 
 import ctypes as C
@@ -35,6 +35,8 @@ def test_panel(lib, n, dtype, cols):
     assert call(p(a), n, cols, p(piv), p(info), C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
     torch.cuda.synchronize()
     assert int(info) == n + 1
+    assert torch.isnan(a[0, 0])
+    a[0, 0] = before[0, 0]
     assert torch.equal(a, before)
     want = np.full(n, -7)
     want[:cols] = np.arange(cols)
