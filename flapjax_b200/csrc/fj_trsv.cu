@@ -16,8 +16,8 @@
 // it only after its warps have applied all but the block before: so when a slot of the ring
 // of solved blocks comes round again, 2 n_cta + 2 <= kRing blocks on, every CTA has done
 // with what it held.
-// Measured, solve (transposed solve) of order 64, 256, 768 and 2048: 12-14, 33, 82 and 210 us
-// (13-14, 35, 87, 221), against 40, 163, 494 and 1324 us (34, 150-168, 467-526, 1305-1434)
+// Measured, solve (transposed solve) of order 64, 256, 768 and 2048: 12-14, 33, 84 and 214 us
+// (13-14, 35, 87, 222), against 40, 163, 494 and 1324 us (34, 150-168, 467-526, 1305-1434)
 // for a launch per diagonal block and per update.  The solving warp's 3,100 to 4,000 cycles
 // per block (column of the triangle: a shuffle's latency in four, then one DFMA's) are what
 // remains on the chain below 768 rows; from 6144 rows (1285 us for 4100) the reading is.
@@ -39,7 +39,7 @@ constexpr int kMaxCtas = 8;
 constexpr int kRing = 20;
 constexpr int kTile = kB * kPitch;
 constexpr int kMaxBuf = 3;           // owned blocks whose tiles are held
-constexpr long long kWaitCycles = 2000000000ll;  // ~1 s at the B200 SM clock
+constexpr long long kWaitCycles = FJ_WAIT_CYCLES;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -64,13 +64,18 @@ struct Shared {
     int dead;
 };
 
-// Waits for a phase, about a second at most; after the first expiry nothing waits.
-__device__ __forceinline__ void wait(Shared& S, const uint64_t& bar, int phase) {
+// Waits for a phase, about a second at most; after the first expiry the CTA waits for nothing, and
+// its solved blocks are NaN.  False unless the phase is complete.
+__device__ __forceinline__ bool wait(Shared& S, const uint64_t& bar, int phase) {
     const uint32_t a = smem_addr(&bar), parity = (uint32_t)phase & 1u;
-    if (try_phase(a, parity)) return;
+    if (kWaitCycles < 0) S.dead = 1;
+    else if (try_phase(a, parity)) return true;
     const long long t0 = clock64();
-    while (!*(volatile int*)&S.dead && !try_phase(a, parity))
+    while (!*(volatile int*)&S.dead) {
+        if (try_phase(a, parity)) return true;
         if (clock64() - t0 > kWaitCycles) S.dead = 1;
+    }
+    return false;
 }
 
 // tile[r][c] = lu[r0 + r][c0 + c], zero outside the matrix; two elements a copy where the
@@ -162,6 +167,17 @@ __device__ __forceinline__ void solve_block(const double* tile, const double* di
     }
 }
 
+// The same by divisions, of a block with a diagonal element whose reciprocal is no normal number;
+// n: the matrix's rows from this block's first.  (Not inlined: rare, and the solving warp's loop stays
+// short.)
+template <bool kTrans>
+__device__ __noinline__ double2 divide_block(const double* tile, double* diag, double2 v, int lane, int n) {
+    for (int r = lane; r < kB; r += 32) diag[r] = r < n ? tile[r * kPitch + r] : 1.0;
+    __syncwarp();
+    solve_block<kTrans, kTrans, kDivisors>(tile, diag, v.x, v.y, lane);
+    return v;
+}
+
 // y -= M x for eight rows, 8 lanes per row: the lane group's rows begin at m and m + 4 stride
 // (null: no such row); x: the lane's eight values.
 template <bool kVec>
@@ -244,27 +260,30 @@ __global__ void __launch_bounds__(kThreads, 1)
             wait(S, S.tiles[k % nbuf], k / nbuf);
             bool divide = false;
             if (!unit) {
-                double d[2];
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int r = lane + 32 * h;
-                    d[h] = b * kB + r < n ? tile[r * kPitch + r] : 1.0;
+                    const double d = b * kB + r < n ? tile[r * kPitch + r] : 1.0;
+                    S.diag[r] = 1.0 / d;
+                    divide = divide || !has_reciprocal(d);
                 }
-                divide = __any_sync(0xffffffffu, !has_reciprocal(d[0]) || !has_reciprocal(d[1]));
-#pragma unroll
-                for (int h = 0; h < 2; ++h) S.diag[lane + 32 * h] = divide ? d[h] : 1.0 / d[h];
+                divide = __any_sync(0xffffffffu, divide);
             }
             __syncwarp();
             wait(S, S.ready, k);
             double* yb = y + b / nc * kB;
             double v0 = yb[lane], v1 = yb[lane + 32];
+            const bool dead = *(volatile int*)&S.dead;
             if (unit) {  // (lower where not transposed, as U is the other way round)
                 solve_block<kTrans, !kTrans, kOnes>(tile, S.diag, v0, v1, lane);
             } else if (divide) {
-                solve_block<kTrans, kTrans, kDivisors>(tile, S.diag, v0, v1, lane);
+                const double2 v = divide_block<kTrans>(tile, S.diag, make_double2(v0, v1), lane, n - b * kB);
+                v0 = v.x;
+                v1 = v.y;
             } else {
                 solve_block<kTrans, kTrans, kReciprocals>(tile, S.diag, v0, v1, lane);
             }
+            if (dead) v0 = v1 = NAN;
             yb[lane] = v0;
             yb[lane + 32] = v1;
             __threadfence_block();  // the update warps meet these rows again in the second substitution
@@ -282,10 +301,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                     : "memory");
             }
             if (!lower) {
-                const double bad = __longlong_as_double(0x7ff8000000000000ll);
-                const bool dead = *(volatile int*)&S.dead;
-                if (b * kB + lane < n) out[b * kB + lane] = dead ? bad : v0;
-                if (b * kB + lane + 32 < n) out[b * kB + lane + 32] = dead ? bad : v1;
+                if (b * kB + lane < n) out[b * kB + lane] = v0;
+                if (b * kB + lane + 32 < n) out[b * kB + lane + 32] = v1;
             }
             ++k;
         }
@@ -316,14 +333,15 @@ __global__ void __launch_bounds__(kThreads, 1)
             prefetch();  // into the buffer of the owned block solved before the last
         };
         if (owned(0)) arrive();
+        bool current = true;  // every phase so far complete: the next may be begun
         for (int t = 0; t + 1 < steps; ++t) {
             const int b = block_of(t), next = block_of(t + 1), slot = t % kRing;
             const bool lower = t < nb;
-            if (u == 0)
+            if (u == 0 && current)
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&S.full[slot])),
                              "n"(kB * 8)
                              : "memory");
-            wait(S, S.full[slot], t / kRing);
+            current = wait(S, S.full[slot], t / kRing) && current;
             double x[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) x[i] = S.x[slot][(lane & 7) * 2 + 16 * (i / 2) + (i & 1)];
@@ -387,6 +405,12 @@ __global__ void __launch_bounds__(kThreads, 1)
                     }
                 }
             }
+        }
+    }
+    if (*(volatile int*)&S.dead) {  // the CTA's own copies and sends arrive first
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        const long long t0 = clock64();
+        while (clock64() - t0 < kSettleCycles) {
         }
     }
     cl.sync();  // no CTA leaves while another may still send to it
