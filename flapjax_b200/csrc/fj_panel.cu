@@ -25,7 +25,7 @@
 //     mbarrier counts, so that no cluster barrier and no fence stand in the chain.  A CTA
 //     sends column j + 2 only after it has every CTA's column j + 1, which each sends after
 //     its last read of column j.  The exchange adds about 450 cycles to a column's 600.
-// Measured, the FP64 LU of order 128, 256, 768 and 2048: 84, 207, 800 and 2600 us, against 187,
+// Measured, the FP64 LU of order 128, 256, 768 and 2048: 88, 209, 797 and 2547 us, against 187,
 // 410, 1480 and 5070 us for lanes that own columns and a cluster barrier per column.  Rows per
 // lane and warps: 4 x 1, 2 x 2 and 1 x 8 were slower for one CTA, 256-row CTAs of a cluster up
 // to 12 %.
@@ -35,7 +35,6 @@
 
 #include <cooperative_groups.h>
 
-#include "fj_bs.cuh"
 #include "fj_panel.cuh"
 
 namespace fj {
@@ -71,13 +70,8 @@ struct Elem<double> {
         if (hi > kInf || (hi == kInf && lo != 0u)) return {1u, 0u};
         return {hi + 2u, lo};
     }
-    // getrf scales by the reciprocal of a pivot that is not subnormal; reciprocal() is for
-    // those whose reciprocal is not subnormal either
-    __device__ static bool fast(uint32_t hi) { return hi - 2u >= 0x00100000u && hi < 0x7fc00000u; }
-    __device__ static double reciprocal(double x) {
-        const double y = rcp_normal(x);
-        return fma(y, fma(-x, y, 1.0), y);  // correctly rounded but for rare halfway cases
-    }
+    // getrf scales by the reciprocal of a pivot that is normal (by hi, of its key)
+    __device__ static bool normal(uint32_t hi) { return hi - 2u >= 0x00100000u; }
 };
 template <>
 struct Elem<float> {
@@ -88,14 +82,7 @@ struct Elem<float> {
         const uint32_t b = lead(x) & 0x7fffffffu;
         return {b > kInf ? 1u : b + 2u, 0u};
     }
-    __device__ static bool fast(uint32_t hi) { return hi - 2u >= 0x00800000u && hi < 0x7e000000u; }
-    __device__ static float reciprocal(float x) {
-        float y;
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-        const float e = fmaf(-x, y, 1.0f);
-        y = fmaf(y, fmaf(e, e, e), y);
-        return fmaf(y, fmaf(-x, y, 1.0f), y);
-    }
+    __device__ static bool normal(uint32_t hi) { return hi - 2u >= 0x00800000u; }
 };
 
 // Columns of the window, and a candidate: its window, and what goes with it.
@@ -294,7 +281,7 @@ __device__ __forceinline__ void columns(T (&v)[RPL][kWin<T>], Rows<RPL>& row, T*
         for (int e = 0; e < RPL; ++e) x[e] = v[e][0];
         T rinv[RPL];
 #pragma unroll
-        for (int e = 0; e < RPL; ++e) rinv[e] = E::reciprocal(x[e]);
+        for (int e = 0; e < RPL; ++e) rinv[e] = T(1) / x[e];
         int num;
         const bool best = search<T, CW, RPL, kCluster>(x, row, S, par, warp, lane, num);
         Cand<T>& mine = kCluster ? S.mine[par] : S.chosen[j - s0];
@@ -338,13 +325,13 @@ __device__ __forceinline__ void columns(T (&v)[RPL][kWin<T>], Rows<RPL>& row, T*
         T l[RPL], lm[RPL];
 #pragma unroll
         for (int i = 0; i < RPL; ++i) lm[i] = l[i] = x[i] * ri;
-        if (!E::fast(h.x)) {  // getrf's operations at the ends of the range; a zero pivot updates nothing
+        if (!E::normal(h.x)) {  // getrf divides by a subnormal pivot; a zero pivot updates nothing
             const T pv = p->row[0];
-            const bool zero = pv == T(0), divide = h.x < E::kInf / 2 || h.x == 1u;
+            const bool zero = pv == T(0);
             if (zero) r = S.zeros;
 #pragma unroll
             for (int i = 0; i < RPL; ++i) {
-                l[i] = zero ? x[i] : divide ? x[i] / pv : x[i] * (T(1) / pv);
+                l[i] = zero ? x[i] : x[i] / pv;
                 lm[i] = zero ? T(0) : l[i];
             }
         }
