@@ -9,8 +9,9 @@
 // and 25 (cutoff) or 26 (epsilon) per filament.
 //   * One reciprocal square root per vertex and one reciprocal per filament.  Both start
 //     from PTX's approximate forms (rsqrt/rcp.approx.ftz.f64, about 20 bits) and take one
-//     third-order Householder step, which cubes the seed's error to below the rounding of
-//     FP64 (tests/test_gpu_pairs.py bounds them against 1 / sqrt and 1 / x).
+//     step of third order by Householder's method (1970), which cubes the seed's error to
+//     below the rounding of FP64: within 1.6 and 1.3 halves of a unit in the last place of
+//     1 / sqrt and 1 / x (tests/test_gpu_pair_functions.py, beside CUDA's own).
 //   * dot = r0.(u1 - u2) as inv1 (r0.r1) - inv2 (r0.r2): no unit vectors.
 //   * The cutoff kernel's radius test |c|^2 > rc^2 |r0|^2 runs on the integer pipe, on the
 //     leading bits of the two sides; pairs within about 1 % of the core radius take the
@@ -26,8 +27,8 @@ namespace fj {
 
 constexpr double kInv4Pi = 1.0 / kFourPi;
 
-// 1 / sqrt(x) for normal x > 0: with h = x y, e = 1 - h y the third-order step is
-// y (1 + e / 2 + 3 e^2 / 8) (Householder, 1970).
+// 1 / sqrt(x) for normal x > 0: with h = x y, e = 1 - h y Householder's step for 1 / y^2 - x is
+// y (1 + e / 2 + 3 e^2 / 8), the binomial series of (1 - e)^(-1/2) to its third term.
 __device__ __forceinline__ double rsqrt_normal(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -35,7 +36,8 @@ __device__ __forceinline__ double rsqrt_normal(double x) {
     return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
-// 1 / x for normal x: y (1 + e + e^2) with e = 1 - x y.
+// 1 / x for normal x below 2^1022: with e = 1 - x y Householder's step for 1 / y - x is y (1 + e + e^2), the
+// geometric series to its third term.
 __device__ __forceinline__ double rcp_normal(double x) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
