@@ -497,8 +497,10 @@ __device__ __forceinline__ void compare_lattice(const StepCase& C, const int64_t
 // alone) want lanes, whose rounds of loads are the time; few (a case's share of a batch) want
 // targets, since what follows keeps one thread in 3 kLanes: k_rhs of one case with 296
 // partials 8.0 us with 16 lanes, 10.6 with 8, 14.6 with 4; k_filaments of 16 cases with 32
-// each 34.5, 22.0 and 14.4 us.  The choice is by a case's own partials, so that it sums in the same
-// order alone and in a batch.
+// each 34.5, 22.0 and 14.4 us (the lines between are drawn from these two).  The choice is by a
+// case's own partials, whose number follows the batch's splits and pieces (see `cut`): a case sums in
+// an order of its own alone and in each batch, equal to 1e-12 in FP64 and 1e-6 in mixed precision
+// (tests/test_gpu_batch.py).
 constexpr int kSumThreads = 384, kSumMinTargets = 8;
 constexpr int kFewPartials = 40, kSomePartials = 128;  // at most: 4 lanes, 8 lanes
 
@@ -1679,7 +1681,7 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
             ref.push_back(rj);
         }
     }
-    // RHS jobs of cases whose wake stream is empty: zero velocity
+    // (a case whose wake stream is empty has no RHS job, and no partials to add)
     assign_splits(jf, precision);
     assign_splits(jr, precision);
     assign_splits(jfo, precision);
@@ -1713,9 +1715,11 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
         return tile;
     };
     const int tf = phase_tile(jf), tr = phase_tile(jr), tfo = phase_tile(jfo);
-    // Each sum's pieces by its own sizes, so that a small case sums in the same order alone and
-    // in a batch; but not where a batch's splits fill the GPU for two waves by themselves (16
-    // wings of up to 12 x 64 panels, FP32: 6030 us in splits alone, 6196 us in pieces as well).
+    // Each sum's pieces by its own sizes and splits, as for a case alone (whose splits, and with
+    // them the order of the sum, are not those of its share in a batch); but not where a batch's
+    // splits fill the GPU for two waves of six CTAs an SM by themselves.  The line is measured for one
+    // FP32 batch at two targets a thread (16 wings of up to 12 x 64 panels: 6030 us in splits alone,
+    // 6196 us in pieces as well) and taken for the other sums as it is.
     auto cut = [&](std::vector<VindJob>& jobs, int prec, int tile) {
         int64_t ctas = 0;
         for (const VindJob& j : jobs) ctas += vind_ctas(j.n_targets, j.n_split, prec, tile);
@@ -1764,9 +1768,9 @@ static int run_steps(std::vector<BatchItem>& items, char* d_tab, size_t tab_byte
     if (sig != nullptr) {
         // Every host value the launches below take outside the table: grid extents, job
         // counts, and the per-case pointers of the launches that are not table-driven (the
-        // FP64 and refactorising solves, the zeroing of cases without far-wake rows).  Two
-        // builds with equal signatures launch the same kernels with the same arguments, so
-        // a graph captured for one replays the other once its table is in place.
+        // FP64 and refactorising solves).  Two builds with equal signatures launch the same
+        // kernels with the same arguments, so a graph captured for one replays the other
+        // once its table is in place.
         std::vector<int64_t>& g = *sig;
         double rc = r_cut;
         int64_t rc_bits = 0;

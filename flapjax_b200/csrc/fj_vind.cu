@@ -437,8 +437,8 @@ __global__ void __launch_bounds__(kBlock, kMinCtas64) vind64_kernel(VindJob job,
 // ------------------------------------------------------------------------------------
 // Packed form: two targets ride in one float2 and every FP32 add/mul/fma of the pair is
 // one f32x2 instruction (sm_100: __fadd2_rn / __fmul2_rn / __ffma2_rn).  Such an instruction
-// takes two issue slots, and the slots bound the sum: 38 (cutoff; epsilon 40) packed ones and
-// 33 others made 109 of the 111 slots a packed pair took.  So the others count as much, and
+// takes two issue slots, and the slots bound the sum: 34 (cutoff; epsilon 36) packed ones and
+// 41 others make 109 of the 113 slots a packed pair takes.  So the others count as much, and
 // what a product by a selected factor would cost in selects a predicated scalar product saves:
 // 25 800 targets x 55 600 filaments, cutoff 2206 -> 2092 us (6.9e11 pairs/s), epsilon 2203 ->
 // 2163 us.  The scalar form, bit for bit the same, has fewer instructions (its negations and
@@ -693,7 +693,7 @@ __device__ __forceinline__ void vind32_body(const double* __restrict__ tgt, int6
 template <int KER, int T>
 __global__ void __launch_bounds__(kBlock, MinCtas32<T>::value) vind32_kernel(VindJob job) {
     vind32_body<KER, T>(job.targets, job.n_targets, (const Elem32*)job.stream, job.n_elem, job.n_split, job.n_sub,
-                        job.part,                         blockIdx.x, blockIdx.y);
+                        job.part, blockIdx.x, blockIdx.y);
 }
 
 // Many jobs in one launch: CTA b belongs to the job j with cta0[j] <= b < cta0[j+1];

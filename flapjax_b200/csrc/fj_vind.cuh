@@ -90,7 +90,7 @@ struct PackJob {
 };
 
 // Batched launches (one kernel for many jobs; tables in device memory).
-//  vind: CTAs of job j are cta0[j] .. cta0[j+1]-1 (ctas_x(j) * n_split(j) of them);
+//  vind: CTAs of job j are cta0[j] .. cta0[j+1]-1 (one per target tile and piece);
 //  all jobs of one launch share precision and kernel.
 // CTAs of a captured launch that replays serve with up to as many (`replayed`).
 int64_t vind_replay_ctas(int64_t total_ctas);
