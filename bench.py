@@ -424,7 +424,7 @@ def main():
             "peak": peak, "unit": "TFLOP/s", "frac": (achieved / peak) if achieved and peak else None,
             "traffic": VIND32_TRAFFIC_BYTES,
             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the convection launch of this "
-                              "workload (profiles/vind32_free_wake_16x128.md); the filament stream is the only "
+                              "workload's size (profiles/pairs_panels_solve.md); the filament stream is the only "
                               "DRAM traffic, the rest stays in L2",
             "peak_source": "measured in-run (fj_peak_fp32: larger of scalar and packed FP32 FMA chains); "
                            "MEASURED_PEAKS.json has no FP32 CUDA-core figure",

@@ -10,7 +10,7 @@
 //     radius of the filament line contribute nothing, derivative included);
 //   * the dense solve (aero/uvlm.py:985) -- A^T mu = lam with the getrf factors of A.
 // K's derivative is in fj_bsgrad.cuh; g_bar = lam.K.
-// 2531 targets x 14 118 filaments (cutoff): targets 419 -> 233 us, filaments 467 -> 313 us, of
+// 2531 targets x 14 118 filaments (cutoff): targets 419 -> 229 us, filaments 467 -> 287 us, of
 // which the FP64 pipe's own 158 and 226 us; 768 x 9 800 (epsilon): 103 -> 63, 106 -> 86 us,
 // against the form with unit vectors and divisions that link_vjp keeps.
 #include <algorithm>
