@@ -67,14 +67,13 @@ struct FilGrad {
 };
 
 // What both derivatives take from a pair: g s, g b, w; s1, s2 = r0.r_i / n_i^2; k = s (lam.c).
-// False for a pair within the core radius, which adds nothing: the callers leave it out, since its
-// other factors may be NaN.
 struct PairGrad {
     double gs, gb, s1, s2, w[3], s, k;
 };
 
-// kFar: den D, of the sixth power of a distance, may leave FP64's range before D and K do: divisions
-// one by one.
+// False for a pair within the core radius, which adds nothing: the callers leave it out, since its
+// other factors may be NaN.  kFar: den D, of the sixth power of a distance, may leave FP64's range
+// before D and K do (from 1e51, where they do from 1e77): divisions one by one.
 template <int KER, bool kFar>
 __device__ __forceinline__ bool pair_grad(const VtxGrad<KER>& A, const VtxGrad<KER>& B, const FilGrad& f, double rc2,
                                           const double lam[3], PairGrad& o) {
